@@ -35,6 +35,7 @@ void free_device(Context* c) {
   // cover composing a batch mesh)
   seg_free(c);
   cg_free(c);
+  resident_reset(c);
   c->d_u_ckpt = c->d_R_ckpt = nullptr;
   c->ckpt_valid = false;
   if (c->pcg_graph) cudaGraphExecDestroy(c->pcg_graph);
@@ -61,6 +62,7 @@ void free_all(Context* c) {
   c->allocations.clear();
   free_templates(c);
   if (c->stream) cudaStreamSynchronize(c->stream);
+  resident_destroy(c);
   if (c->h_pcg) cudaFreeHost(c->h_pcg);
   if (c->h_resid) cudaFreeHost(c->h_resid);
   if (c->h_status) cudaFreeHost(c->h_status);
@@ -187,6 +189,7 @@ int alloc_mesh(Context* c, int nnd, int nel, int neq, long long nnzb) {
   c->have_blocks = false;
   c->have_du = false;
   c->composed = false;
+  c->inst_segments = false;
   c->h_conn.clear();
   c->h_eqnos.clear();
   c->h_coords.clear();

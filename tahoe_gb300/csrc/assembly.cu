@@ -18,89 +18,18 @@
 // (minv_diag_offset).
 #include <type_traits>
 
-#include "tg_internal.h"
+#include "assembly.cuh"
 
 namespace tg {
 
 namespace {
 
-__device__ __forceinline__ int upper_slot(int a, int b) { return a * 8 - a * (a - 1) / 2 + (b - a); }
-
-// The value of global block j: its element contributions in the
-// destination-sorted order, rows of prescribed dofs zeroed (columns are kept,
-// so a product with a prescribed-increment vector gives the coupling
-// K_fp du_p; PCG vectors are zero at prescribed dofs, so the kept columns
-// never enter the solve).
-template <typename T>
-__device__ __forceinline__ void block_value(int j, uint8_t mI, const int* __restrict__ cptr,
-                                            const int* __restrict__ contrib, const T* __restrict__ Ke, T acc[9]) {
-  using V4 = typename std::conditional<sizeof(T) == 4, float4, double4_32a>::type;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) acc[k] = T(0);
-  const int c1 = cptr[j + 1];
-  for (int c = cptr[j]; c < c1; ++c) {
-    const int code = contrib[c];
-    const int e = code >> 6, a = (code >> 3) & 7, b = code & 7;
-    // the element block's three padded rows: one aligned vector load each
-    const V4* src = reinterpret_cast<const V4*>(
-        Ke + ((long long)e * kSlots + (a <= b ? upper_slot(a, b) : upper_slot(b, a))) * kKeBlock);
-    const V4 k0 = src[0], k1 = src[1], k2 = src[2];
-    const T m[9] = {k0.x, k0.y, k0.z, k1.x, k1.y, k1.z, k2.x, k2.y, k2.z};
-    if (a <= b) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) acc[k] += m[k];
-    } else {
-#pragma unroll
-      for (int p = 0; p < 3; ++p)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) acc[p * 3 + q] += m[q * 3 + p];
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < 3; ++p)
-    if (!((mI >> p) & 1))
-#pragma unroll
-      for (int q = 0; q < 3; ++q) acc[p * 3 + q] = T(0);
-}
-
-// (block-)Jacobi inverse of row I's diagonal block; inactive dofs get
-// identity in the inverse's input and zero in its output.
+// the inverses of row I's diagonal block into the preconditioner storage
 template <typename T>
 __device__ __forceinline__ void write_inverses(int I, int nnd, uint8_t mI, const T acc[9], T* __restrict__ minv) {
   using V4 = typename std::conditional<sizeof(T) == 4, float4, double4_32a>::type;
-  T A[9];
-#pragma unroll
-  for (int p = 0; p < 3; ++p)
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-      A[p * 3 + q] = (((mI >> p) & 1) && ((mI >> q) & 1)) ? acc[p * 3 + q] : (p == q ? T(1) : T(0));
-  // Jacobi: inverse diagonal; block-Jacobi: inverse of the 3x3 block
-  T B[9], Dg[9];
-  const T d = A[0] * (A[4] * A[8] - A[5] * A[7]) - A[1] * (A[3] * A[8] - A[5] * A[6]) +
-              A[2] * (A[3] * A[7] - A[4] * A[6]);
-  const T id = T(1) / d;
-  B[0] = (A[4] * A[8] - A[5] * A[7]) * id;
-  B[1] = (A[2] * A[7] - A[1] * A[8]) * id;
-  B[2] = (A[1] * A[5] - A[2] * A[4]) * id;
-  B[3] = (A[5] * A[6] - A[3] * A[8]) * id;
-  B[4] = (A[0] * A[8] - A[2] * A[6]) * id;
-  B[5] = (A[2] * A[3] - A[0] * A[5]) * id;
-  B[6] = (A[3] * A[7] - A[4] * A[6]) * id;
-  B[7] = (A[1] * A[6] - A[0] * A[7]) * id;
-  B[8] = (A[0] * A[4] - A[1] * A[3]) * id;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) Dg[k] = T(0);
-  Dg[0] = T(1) / A[0];
-  Dg[4] = T(1) / A[4];
-  Dg[8] = T(1) / A[8];
-#pragma unroll
-  for (int p = 0; p < 3; ++p)
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-      if (!((mI >> p) & 1) || !((mI >> q) & 1)) {
-        B[p * 3 + q] = T(0);
-        Dg[p * 3 + q] = T(0);
-      }
+  T Dg[9], B[9];
+  diagonal_inverses<T>(mI, acc, Dg, B);
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     minv[(long long)I * 9 + k] = Dg[k];
@@ -170,6 +99,57 @@ __global__ void __launch_bounds__(256) assemble_upper_kernel(
       for (int k = 0; k < 9; ++k) planes[(long long)k * ps + kr + (j - jd)] = acc[k];
       if (j == jd) write_inverses<T>(I, nnd, mI, acc, minv);
     }
+  }
+}
+
+// rhs = R - K v on the active rows from the element blocks, accumulated in
+// FP64 (v a prescribed increment, zero on free dofs): eight lanes per node,
+// lane b multiplies column b of every incident element whose node b carries a
+// prescribed dof.  The rows away from the prescribed nodes read no blocks, so
+// no assembled matrix is needed (the predictor of a batch spent more time on
+// assembling the full storage for this product than on the product).
+template <typename T>
+__global__ void __launch_bounds__(256) lift_elements_kernel(
+    int nnd, const int* __restrict__ nptr, const int* __restrict__ nlist, const int* __restrict__ conn,
+    const uint8_t* __restrict__ mask, const T* __restrict__ Ke, const double4_32a* __restrict__ v,
+    const double4_32a* __restrict__ R, double4_32a* __restrict__ rhs) {
+  using V4 = typename std::conditional<sizeof(T) == 4, float4, double4_32a>::type;
+  const int b = threadIdx.x & 7;
+  const int I = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3);
+  if (I - (int)((threadIdx.x & 31) >> 3) >= nnd) return;  // whole warps
+  const uint8_t m = I < nnd ? mask[I] : 0;
+  double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+  if (m) {
+    const int k1 = nptr[I + 1];
+    for (int k = nptr[I]; k < k1; ++k) {
+      const int code = nlist[k], e = code >> 3, a = code & 7;
+      const int n = conn[e * 8 + b];
+      if (mask[n] == 7) continue;
+      const double4_32a vn = v[n];
+      if (vn.x == 0.0 && vn.y == 0.0 && vn.z == 0.0) continue;
+      const V4* src = reinterpret_cast<const V4*>(
+          Ke + ((long long)e * kSlots + (a <= b ? upper_slot(a, b) : upper_slot(b, a))) * kKeBlock);
+      const V4 k0 = src[0], k1r = src[1], k2 = src[2];
+      if (a <= b) {
+        a0 += (double)k0.x * vn.x + (double)k0.y * vn.y + (double)k0.z * vn.z;
+        a1 += (double)k1r.x * vn.x + (double)k1r.y * vn.y + (double)k1r.z * vn.z;
+        a2 += (double)k2.x * vn.x + (double)k2.y * vn.y + (double)k2.z * vn.z;
+      } else {
+        a0 += (double)k0.x * vn.x + (double)k1r.x * vn.y + (double)k2.x * vn.z;
+        a1 += (double)k0.y * vn.x + (double)k1r.y * vn.y + (double)k2.y * vn.z;
+        a2 += (double)k0.z * vn.x + (double)k1r.z * vn.y + (double)k2.z * vn.z;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+    a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+    a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+  }
+  if (I < nnd && b == 0) {
+    const double4_32a r = R[I];
+    rhs[I] = make_double4_32a(r.x - ((m & 1) ? a0 : 0.0), r.y - ((m & 2) ? a1 : 0.0), r.z - ((m & 4) ? a2 : 0.0), 0.0);
   }
 }
 
@@ -327,6 +307,18 @@ int ensure_full_assembly(Context* c) {
   if (!s) s = launch_assemble(c, precision);
   if (!s) serial = c->tangent_serial;
   return s;
+}
+
+int launch_lift_elements(Context* c, const double4_32a* d_v, double4_32a* d_rhs) {
+  const int grid = (int)(((long long)c->nnd * 8 + 255) / 256);
+  if (c->tangent_precision == TG_MIXED)
+    lift_elements_kernel<float><<<grid, 256, 0, c->stream>>>(c->nnd, c->d_node_elem_ptr, c->d_node_elem, c->d_conn,
+                                                             c->d_mask, c->d_Ke32, d_v, c->d_R, d_rhs);
+  else
+    lift_elements_kernel<double><<<grid, 256, 0, c->stream>>>(c->nnd, c->d_node_elem_ptr, c->d_node_elem, c->d_conn,
+                                                              c->d_mask, c->d_Ke64, d_v, c->d_R, d_rhs);
+  c->launches++;
+  return ok(c, cudaGetLastError(), "lift_elements_kernel") ? TG_OK : TG_ERR_CUDA;
 }
 
 int launch_set_prescribed(Context* c, int n, const int* d_idx, const double* d_val) {

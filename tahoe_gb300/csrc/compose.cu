@@ -13,7 +13,7 @@
 #include <string>
 #include <vector>
 
-#include "tg_internal.h"
+#include "respcg.cuh"
 
 namespace tg {
 
@@ -36,7 +36,15 @@ struct TplDev {
 
 struct MeshTemplate {
   TplDev dev{};
-  std::vector<int> rowptr;      // host block-row pointers (re-tiling)
+  std::vector<int> rowptr;      // host block-row pointers (re-tiling, resident rows)
+  std::vector<int> col;         // host block columns and active-dof bits (resident rows)
+  std::vector<uint8_t> mask;
+  // resident PCG: the rows, their device copy and one split per precision
+  ResRows res_rows;
+  ResPlanDev res_dev{};
+  bool res_built = false;
+  int res_state[2] = {0, 0};    // 0 not planned, 1 fits, -1 does not
+  ResPlan res_plan[2];
   std::vector<int> tile_row;    // local tile starts, ntiles+1
   std::vector<long long> tile_b32, tile_b64;  // bytes of every tile in the tile-contiguous storage
   int tile_blocks = 0;
@@ -234,6 +242,63 @@ int template_geometry_pool(Context* c, TplGeoPool& pool) {
 template int template_geometry_pool<float2>(Context*, TplGeoPool&);
 template int template_geometry_pool<double>(Context*, TplGeoPool&);
 
+// A template's resident rows and their split for one precision, kept with the
+// template: every batch composed from it uses them.
+int template_resident(Context* c, int tpl, int precision, ResPlan& P, bool& fits) {
+  MeshTemplate* t = c->templates[tpl];
+  const int p = precision == TG_MIXED ? 1 : 0;
+  fits = false;
+  auto put = [&](const ResImage& img, int** d) {
+    if (!talloc(c, t, d, img.data.size())) return TG_ERR_OOM;
+    return ok(c, cudaMemcpyAsync(*d, img.data.data(), sizeof(int) * img.data.size(), cudaMemcpyHostToDevice, c->stream),
+              "resident rows") &&
+                   ok(c, cudaStreamSynchronize(c->stream), "sync")
+               ? TG_OK
+               : TG_ERR_CUDA;
+  };
+  if (!t->res_built) {
+    resident_rows(0, t->dev.nnd, t->rowptr.data(), t->col.data(), t->mask.data(), t->res_rows);
+    ResImage img;
+    const size_t at = img.rows_at(t->res_rows);
+    int* d = nullptr;
+    const int s = put(img, &d);
+    if (s) return s;
+    resident_bind_rows(t->res_dev, d, at, t->res_rows);
+    t->res_dev.contrib = t->dev.contrib;
+    int2* slot = nullptr;
+    if (!talloc(c, t, &slot, t->res_rows.blk.size())) return TG_ERR_OOM;
+    t->res_dev.slot = slot;
+    const int ss = resident_slots(c, (long long)t->res_rows.blk.size(), t->res_dev.blk, t->dev.cptr, slot);
+    if (ss) return ss;
+    t->res_built = true;
+  }
+  if (t->res_state[p] == 0) {
+    size_t cap = 0;
+    int cluster = 1;
+    int s = resident_limits(c, precision, &cap, &cluster);
+    if (s) return s;
+    ResPlan& Q = t->res_plan[p];
+    Q = ResPlan{};
+    if (t->res_rows.act_node.empty()) {
+      t->res_state[p] = 1;  // nothing to solve
+    } else if (resident_plan(t->res_rows, p ? 4 : 8, c->num_sms, cap, cluster, false, Q)) {
+      ResImage img;
+      const size_t at = img.split_at(Q);
+      int* d = nullptr;
+      s = put(img, &d);
+      if (s) return s;
+      Q.dev = t->res_dev;
+      resident_bind_split(Q.dev, d, at, Q);
+      t->res_state[p] = 1;
+    } else {
+      t->res_state[p] = -1;
+    }
+  }
+  fits = t->res_state[p] > 0;
+  if (fits) P = t->res_plan[p];
+  return TG_OK;
+}
+
 int launch_affine_prescribed(Context* c, const double* d_F) {
   affine_prescribed_kernel<<<(c->nnd + 255) / 256, 256, 0, c->stream>>>(c->nnd, c->nseg, c->d_seg_node, d_F, c->d_X,
                                                                          c->d_mask, c->d_u);
@@ -362,6 +427,8 @@ int tg_template_add(tg_context* c, int nnd, const double* coords, int nel, const
     delete t;
     return st;
   }
+  t->col.swap(col);
+  t->mask.swap(mask);
   *template_id = (int)c->templates.size();
   c->templates.push_back(t);
   c->tpl_elems += nel;
@@ -452,6 +519,7 @@ int tg_mesh_compose(tg_context* c, int count, const int* template_ids) {
   dfree(c, d_tpl);
   dfree(c, d_inst);
   c->have_blocks = true;
+  c->inst_segments = true;
   c->nseg = count;
   c->h_seg_node.resize(count + 1);
   c->h_seg_elem.resize(count + 1);

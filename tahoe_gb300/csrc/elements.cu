@@ -1226,6 +1226,7 @@ int launch_element_dump(Context* c, int first, int count, double* dKe, double* d
   int s = c->tangent_precision == TG_FP64 ? ensure_full_assembly(c) : TG_OK;
   if (!s) s = residual_impl(c, 0);
   if (s) return s;
+  c->ke_serial64 = -1;
   s = launch_tangent(c, TG_FP64);
   if (s) return s;
   expand_ke_kernel<<<count, 256, 0, c->stream>>>(first, count, c->d_Ke64, c->d_fint, dKe, dfint);

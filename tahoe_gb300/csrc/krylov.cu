@@ -864,8 +864,12 @@ int time_pcg_t(Context* c, int which, int reps, double* ms) {
 }
 
 int time_pcg_kernel(Context* c, int which, int reps, double* ms) {
-  // the kernels the solve runs: the single-reduction form's own pair, or
-  // the product of a segmented batch on the push storage
+  // the streamed kernels: the single-reduction form's own pair, or the
+  // product of a segmented batch on the push storage
+  if (c->tangent_precision >= 0) {
+    const int sf = push_solve(c) ? push_prepare(c, c->tangent_precision) : ensure_full_assembly(c);
+    if (sf) return sf;
+  }
   if (c->nseg > 0 && which == 0 && push_active(c)) return time_seg_push(c, reps, ms);
   if (c->pcg_form == 1 && !sym_active(c) && c->nseg == 0) return time_cg_kernel(c, which, reps, ms);
   if (c->tangent_precision == TG_MIXED) return time_pcg_t<float>(c, which, reps, ms);
@@ -999,9 +1003,16 @@ void spmv_run(Context* c, int precision, const SpmvPlan& P, const void* p, void*
 
 int pcg_solve(Context* c, const double4_32a* d_rhs, double rel_tol, int max_it, int precond, int* iters,
               double* rel_res) {
-  // a solve that streams the full storage: its values from the last tangent
-  if (!push_solve(c)) {
-    const int sf = ensure_full_assembly(c);
+  if (ke_current(c)) {
+    bool resident = false;
+    const int sr = resident_active(c, c->tangent_precision, &resident);
+    if (sr) return sr;
+    if (resident) return pcg_solve_resident(c, d_rhs, rel_tol, max_it, precond, iters, rel_res);
+  }
+  // a solve that streams a matrix storage: its values (and the
+  // preconditioner's) from the last tangent
+  {
+    const int sf = push_solve(c) ? push_prepare(c, c->tangent_precision) : ensure_full_assembly(c);
     if (sf) return sf;
   }
   // a batch of RVEs: one Krylov solve per RVE over the shared matrix stream

@@ -105,7 +105,12 @@ int form_tangent(Context* c, int precision) {
     if (!c->d_minv64 && !dalloc(c, &c->d_minv64, minv_values(c->nnd))) return TG_ERR_OOM;
   }
   int s = launch_tangent(c, precision);
-  if (!s && push_solve(c)) {
+  bool resident = false;
+  if (!s) s = resident_active(c, precision, &resident);
+  if (!s && resident) {
+    // the solve assembles its rows from the element blocks itself
+    ++c->tangent_serial;
+  } else if (!s && push_solve(c)) {
     // the solve streams the push storage: its upper blocks are assembled
     // straight into it, the full storage only when something reads it
     s = launch_assemble_upper(c, precision);
@@ -123,6 +128,7 @@ int form_tangent(Context* c, int precision) {
     // the symmetric stream format of the single-vector product
     if (!s && sym_active(c)) s = sym_convert(c, precision);
   }
+  if (!s) (precision == TG_MIXED ? c->ke_serial32 : c->ke_serial64) = c->tangent_serial;
   if (!s) s = check_status(c);
   if (!s) c->tangent_precision = precision;
   return s;
@@ -557,7 +563,7 @@ int predict(tg_context* c, int n, const int* idx, const double* val, const doubl
   // u now carries the new prescribed values
   if (!s) s = F ? launch_affine_prescribed(c, d_val) : launch_set_prescribed(c, n, d_idx, d_val);
   if (!s) s = launch_diff(c, c->d_u, d_old, d_v);         // v = du_p (zero on free dofs)
-  if (!s) s = launch_lift_rhs(c, d_v, d_old);             // rhs = R - K v (d_old is free after the diff)
+  if (!s) s = launch_lift_elements(c, d_v, d_old);        // rhs = R - K v (d_old is free after the diff)
   int its = 0;
   double rr = 0.0;
   if (!s) {
@@ -596,6 +602,8 @@ int tg_set_segments(tg_context* c, int nseg, const int* node_off, const int* ele
     *p = nullptr;
   }
   seg_free(c);  // the per-RVE solve's chunks follow the partition
+  resident_drop_batch(c);
+  c->inst_segments = false;
   c->nseg = nseg;
   c->h_seg_node.assign(node_off, node_off + nseg + 1);
   c->h_seg_elem.assign(elem_off, elem_off + nseg + 1);
@@ -818,6 +826,13 @@ int tg_time_kernel(tg_context* c, int which, int reps, double* ms) {
   if ((which == 2 || which == 3) && c->tangent_precision < 0) {
     c->err = "form a tangent first (its precision is the one timed)";
     return TG_ERR_ARG;
+  }
+  if (which == 2) {
+    // the element blocks are re-formed at the current state: the tangent's
+    // own assembly comes first, and its blocks are no longer on the device
+    const int sf = ensure_full_assembly(c);
+    if (sf) return sf;
+    (c->tangent_precision == TG_MIXED ? c->ke_serial32 : c->ke_serial64) = -1;
   }
   cudaEvent_t a, b;
   cudaEventCreate(&a);

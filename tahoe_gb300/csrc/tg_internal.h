@@ -71,6 +71,7 @@ struct ResidScalars {
   int pad;
 };
 
+struct ResState;      // plans and buffers of the resident PCG (respcg.cuh)
 struct MeshTemplate;  // a resident template mesh (compose.cu)
 // geometry planes (25 planes of 8 points per element) of every resident
 // template: the element-major offsets are the templates' pool offsets
@@ -239,6 +240,8 @@ struct Context {
   // product amortises its build; the full storage below)
   int cg_push = -1;
   long long tangent_serial = 0; // assemblies so far (values of derived storages follow it)
+  long long ke_serial32 = -1, ke_serial64 = -1;      // tangent serial of the element blocks on the device
+  ResState* res = nullptr;
   long long full_serial32 = -1, full_serial64 = -1;  // tangent serial of the full storage's values
   int* d_contrib_ptr = nullptr; // nnzb+1
   int* d_contrib = nullptr;     // nel*64: e*64 + a*8 + b
@@ -336,6 +339,7 @@ struct Context {
   TplGeoPool tpl_geo_ff, tpl_geo64;
   long long tpl_elems = 0;      // elements of every template added (pool offsets, append-only)
   bool composed = false;           // mesh built by tg_mesh_compose (host copies on demand)
+  bool inst_segments = false;      // its RVEs are its instances (no other partition was set)
   std::vector<int> h_inst_tpl;     // template of every instance of the composed mesh
 
   std::vector<void*> allocations;
@@ -466,6 +470,20 @@ int pcg_finish(Context* c, const PcgScalars& h, int* iters, double* rel_res);
 int pcg_solve_cg(Context* c, int precision, const double4_32a* d_rhs, double rel_tol, int max_it, int precond,
                  int* iters, double* rel_res);
 void cg_free(Context* c);  // the captured iterations
+// resident PCG (respcg.cu): whether the next solve of the given precision runs
+// it (plans the mesh on first use), the solve, and what it keeps per mesh
+int resident_active(Context* c, int precision, bool* on);
+int pcg_solve_resident(Context* c, const double4_32a* d_rhs, double rel_tol, int max_it, int precond, int* iters,
+                       double* rel_res);
+void resident_reset(Context* c);
+void resident_drop_batch(Context* c);
+void resident_destroy(Context* c);
+inline bool ke_current(const Context* c) {
+  return (c->tangent_precision == TG_MIXED && c->ke_serial32 == c->tangent_serial) ||
+         (c->tangent_precision == TG_FP64 && c->ke_serial64 == c->tangent_serial);
+}
+// rhs = R - K v from the element blocks, v zero away from prescribed dofs
+int launch_lift_elements(Context* c, const double4_32a* d_v, double4_32a* d_rhs);
 // symmetric push storage: structure (once per mesh) and values of the last
 // assembly in the given precision (pushfmt.cu)
 int push_prepare(Context* c, int precision);
