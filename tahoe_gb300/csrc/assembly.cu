@@ -111,8 +111,11 @@ __global__ void __launch_bounds__(256) assemble_upper_kernel(
 template <typename T>
 __global__ void __launch_bounds__(256) lift_elements_kernel(
     int nnd, const int* __restrict__ nptr, const int* __restrict__ nlist, const int* __restrict__ conn,
-    const uint8_t* __restrict__ mask, const T* __restrict__ Ke, const double4_32a* __restrict__ v,
-    const double4_32a* __restrict__ R, double4_32a* __restrict__ rhs) {
+    const uint8_t* __restrict__ mask, const T* __restrict__ Ke, const double4_32a* __restrict__ v_all,
+    const double4_32a* __restrict__ R, double4_32a* __restrict__ rhs_all) {
+  // grid rows (blockIdx.y) are independent vectors v, rhs (nnd apart)
+  const double4_32a* __restrict__ v = v_all + (long long)blockIdx.y * nnd;
+  double4_32a* __restrict__ rhs = rhs_all + (long long)blockIdx.y * nnd;
   using V4 = typename std::conditional<sizeof(T) == 4, float4, double4_32a>::type;
   const int b = threadIdx.x & 7;
   const int I = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3);
@@ -148,7 +151,7 @@ __global__ void __launch_bounds__(256) lift_elements_kernel(
     a2 += __shfl_xor_sync(0xffffffffu, a2, o);
   }
   if (I < nnd && b == 0) {
-    const double4_32a r = R[I];
+    const double4_32a r = R ? R[I] : make_double4_32a(0.0, 0.0, 0.0, 0.0);
     rhs[I] = make_double4_32a(r.x - ((m & 1) ? a0 : 0.0), r.y - ((m & 2) ? a1 : 0.0), r.z - ((m & 4) ? a2 : 0.0), 0.0);
   }
 }
@@ -309,14 +312,15 @@ int ensure_full_assembly(Context* c) {
   return s;
 }
 
-int launch_lift_elements(Context* c, const double4_32a* d_v, double4_32a* d_rhs) {
-  const int grid = (int)(((long long)c->nnd * 8 + 255) / 256);
+int launch_lift_elements(Context* c, const double4_32a* d_v, double4_32a* d_rhs, bool zero_base, int nvec) {
+  const dim3 grid((unsigned)(((long long)c->nnd * 8 + 255) / 256), (unsigned)nvec);
+  const double4_32a* R = zero_base ? nullptr : c->d_R;
   if (c->tangent_precision == TG_MIXED)
     lift_elements_kernel<float><<<grid, 256, 0, c->stream>>>(c->nnd, c->d_node_elem_ptr, c->d_node_elem, c->d_conn,
-                                                             c->d_mask, c->d_Ke32, d_v, c->d_R, d_rhs);
+                                                             c->d_mask, c->d_Ke32, d_v, R, d_rhs);
   else
     lift_elements_kernel<double><<<grid, 256, 0, c->stream>>>(c->nnd, c->d_node_elem_ptr, c->d_node_elem, c->d_conn,
-                                                              c->d_mask, c->d_Ke64, d_v, c->d_R, d_rhs);
+                                                              c->d_mask, c->d_Ke64, d_v, R, d_rhs);
   c->launches++;
   return ok(c, cudaGetLastError(), "lift_elements_kernel") ? TG_OK : TG_ERR_CUDA;
 }

@@ -621,8 +621,14 @@ int mrhs_solve_t(Context* c, const double4_32a* d_b, const double4_32a* d_v, dou
 // formed at the current state.
 int macro_tangent_mrhs(Context* c, int precision, int precond, double rel_tol, int max_it, const double* d_vol,
                        double* d_C, int* iters) {
-  {
-    // the multi-vector product streams the full storage
+  // RVEs that the default form solves resident: nine solves of each, side by
+  // side; else one multi-vector PCG over the batch on the full storage
+  bool resident = false;
+  if (c->seg_pcg_mode && ke_current(c)) {
+    const int sr = resident_active(c, precision, &resident);
+    if (sr) return sr;
+  }
+  if (!resident) {
     const int sf = ensure_full_assembly(c);
     if (sf) return sf;
   }
@@ -634,9 +640,12 @@ int macro_tangent_mrhs(Context* c, int precision, int precond, double rel_tol, i
   int s = TG_OK;
   // boundary perturbations v_kL = (e_k (x) e_L) X and right-hand sides -K v
   for (int kL = 0; kL < kNR && !s; ++kL) s = launch_macro_perturb(c, kL / 3, kL % 3, d_v + (size_t)kL * c->nnd);
-  if (!s) s = launch_lift_rhs(c, d_v, d_b, true, kNR);
+  if (!s) s = resident ? launch_lift_elements(c, d_v, d_b, true, kNR) : launch_lift_rhs(c, d_v, d_b, true, kNR);
   double worst = 0.0;
-  if (!s) {
+  if (!s && resident) {
+    s = macro_solve_resident(c, precision, kNR, d_b, d_v, d_b, rel_tol, max_it, precond, iters);
+    if (s == TG_ERR_NOT_CONVERGED) s = TG_OK;
+  } else if (!s) {
     s = precision == TG_MIXED ? mrhs_solve_t<float>(c, d_b, d_v, d_b, rel_tol, max_it, precond, iters, &worst)
                               : mrhs_solve_t<double>(c, d_b, d_v, d_b, rel_tol, max_it, precond, iters, &worst);
     if (s == TG_ERR_NOT_CONVERGED) s = TG_OK;

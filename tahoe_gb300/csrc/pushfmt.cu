@@ -288,17 +288,6 @@ __global__ void __launch_bounds__(256) push_convert_kernel(
   }
 }
 
-int launch_scan(Context* c, int n, const int* d_in, int* d_out, int* d_tmp) {
-  const int nblk = (n + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems);
-  int* bsum = d_tmp;
-  int* total = d_tmp + std::max(nblk, 1);
-  if (nblk > 0) scan_block_kernel<<<nblk, kScanThreads, 0, c->stream>>>(n, d_in, d_out, bsum);
-  scan_sums_kernel<<<1, kScanThreads, 0, c->stream>>>(nblk, bsum, total);
-  scan_add_kernel<<<(n + 256) / 256, 256, 0, c->stream>>>(n, bsum, total, d_out);
-  c->launches += 3;
-  return ok(c, cudaGetLastError(), "scan") ? TG_OK : TG_ERR_CUDA;
-}
-
 int push_build(Context* c) {
   PushStore& ps = c->push;
   push_free(c);
@@ -328,8 +317,8 @@ int push_build(Context* c) {
     c->launches++;
     if (!ok(c, cudaGetLastError(), "push_count_kernel")) s = TG_ERR_CUDA;
   }
-  if (!s) s = launch_scan(c, n, d_ucnt, ps.d_urow, d_tmp);
-  if (!s) s = launch_scan(c, n, d_lcnt, ps.d_lptr, d_tmp);
+  if (!s) s = scan_counts(c, n, d_ucnt, ps.d_urow, d_tmp);
+  if (!s) s = scan_counts(c, n, d_lcnt, ps.d_lptr, d_tmp);
   int h_flag[2] = {0, 0}, nu = 0, nl = 0;
   if (!s && (!ok(c, cudaMemcpyAsync(h_flag, d_flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, st), "flag") ||
              !ok(c, cudaMemcpyAsync(&nu, ps.d_urow + n, sizeof(int), cudaMemcpyDeviceToHost, st), "nu") ||
@@ -443,6 +432,18 @@ int push_blob(Context* c, int precision) {
 }
 
 }  // namespace
+
+// exclusive scan of n counts into out[0..n]; tmp holds the block sums
+int scan_counts(Context* c, int n, const int* d_in, int* d_out, int* d_tmp) {
+  const int nblk = (n + kScanThreads * kScanItems - 1) / (kScanThreads * kScanItems);
+  int* bsum = d_tmp;
+  int* total = d_tmp + std::max(nblk, 1);
+  if (nblk > 0) scan_block_kernel<<<nblk, kScanThreads, 0, c->stream>>>(n, d_in, d_out, bsum);
+  scan_sums_kernel<<<1, kScanThreads, 0, c->stream>>>(nblk, bsum, total);
+  scan_add_kernel<<<(n + 256) / 256, 256, 0, c->stream>>>(n, bsum, total, d_out);
+  c->launches += 3;
+  return ok(c, cudaGetLastError(), "scan") ? TG_OK : TG_ERR_CUDA;
+}
 
 int push_structure(Context* c, int precision) {
   PushStore& ps = c->push;

@@ -58,25 +58,33 @@ namespace tg {
 namespace {
 
 constexpr int kResClusterMax = 16;
+constexpr int kResCopies = 16;         // tables of the CTAs' sums (grid form)
 constexpr int kResPollLimit = 1 << 21;  // polls of one exchange word before the solve is abandoned
 
-// Shape of a CTA: warps, chunks of 8 rows per warp at most, and the steps of
-// a warp's first chunk whose blocks stay in registers.  FP32: 16 warps at 128
-// registers keep 16 chunks in registers beside the 27 that fit the shared
-// memory, so a solve takes about 0.6 of the CTAs that shared memory alone
-// would ask for; a chip's clusters are few when they are large (13 of 10
-// CTAs, 8 of 11 or 12, 7 of 13 to 16).  FP64 runs at the rate of the FP64
-// pipe (one warp instruction per 64 cycles and scheduler), not of the storage.
+// Shape of a CTA: warps, chunks of 8 rows per warp at most, and for a warp's
+// first `off` chunks the steps whose blocks stay out of shared memory.
+//
+// FP32: 16 warps at 128 registers.  A warp's first chunk keeps seven steps (27
+// blocks a row) in registers, its second and third in tensor memory, the
+// fourth in shared memory, so a CTA holds 64 chunks where shared memory alone
+// held 26: the SM's tensor memory is 256 KB that this solve's warps read
+// beside the shared-memory pipe (a step costs that pipe 5 wavefronts from
+// registers or tensor memory, its column indices and gathered vectors, and 14
+// from shared memory).  Fewer CTAs a solve also means more solves at once: a
+// chip runs 46 clusters of 3 CTAs, 28 of 5, 15 of 7 to 9, 8 of 11 or 12.
+// FP64 runs at the rate of the FP64 pipe (one warp instruction per 64 cycles
+// and scheduler), not of the storage: shared memory alone.
 template <typename T>
 struct ResShape;
 template <>
 struct ResShape<float> {
-  static constexpr int warps = 16, slots = 3, reg = 7;
+  static constexpr int warps = 16, slots = 4, reg = 7, off = 3, state = 6;
 };
 template <>
 struct ResShape<double> {
-  static constexpr int warps = 16, slots = 1, reg = 0;
+  static constexpr int warps = 16, slots = 1, reg = 0, off = 0, state = 0;
 };
+constexpr int kTmemColumns = 512;
 
 using u64 = unsigned long long;
 
@@ -189,6 +197,43 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, unsigned parity
   return false;
 }
 
+// Tensor memory as plain storage: a warp reads and writes the 32 lanes of its
+// quarter, one 32-bit value per thread and column.
+__device__ __forceinline__ void tmem_alloc(unsigned* at) {
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(at)),
+               "n"(kTmemColumns)
+               : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+}
+__device__ __forceinline__ void tmem_free(unsigned addr) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "n"(kTmemColumns));
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_st9(unsigned a, const float* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(a),
+               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+               "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+               "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+               : "memory");
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(a + 8u), "r"(__float_as_uint(v[8])) : "memory");
+}
+__device__ __forceinline__ void tmem_ld9(unsigned a, unsigned* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(a));
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v[8]) : "r"(a + 8u));
+}
+__device__ __forceinline__ void tmem_ld18(unsigned a, unsigned* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(a));
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(v[16]), "=r"(v[17]) : "r"(a + 16u));
+}
+
 template <typename T>
 struct ResArgs {
   const ResPlanDev* plans;
@@ -205,6 +250,7 @@ struct ResArgs {
   PcgScalars* sc;        // receives unscale (single solve) or 1 (batch)
   int* status;
   int batch;             // the solution is unscaled in place
+  int nnd;               // nodes of one right-hand side and solution
   int max_it;
   double tol;
 };
@@ -217,38 +263,102 @@ struct ResShared {
   int4 peer[kResClusterMax];         // {first column, columns, window address, bar_u address} of every part
   u64 red[3][16 * 8];                // sums of every row quad of lanes
   u64 slot[2][kResClusterMax][3];    // the CTAs' sums by parity
+  u64 part[3][8];                    // grid form: sums of the polling warps
   u64 tot[3];                        // totals
   T coef[2];                         // alpha, beta
-  // the recurrence's scalars (thread 0): gamma and alpha of the last update,
-  // convergence threshold, r.r now and at the start
+  // the recurrence's scalars: gamma and alpha of the last update (FP32: 1 /
+  // (gamma alpha) and 1 / gamma), convergence threshold, r.r now and at the start
   u64 rz, al, thr, rr, rr0;
   int code, fail;
   int abort_flag;
+  unsigned tmem;                     // the CTA's tensor memory
 };
 
-// Totals of three accumulators over every row of the solve, left in sh.tot:
-// lanes, warps and CTAs in a fixed order.  seq numbers the reductions of a
-// solve from 1.  On return warp 0 sees sh.tot.
+// Totals of three accumulators over every row of the solve, returned to
+// thread 0 (and left in sh.tot): lanes, warps and CTAs in a fixed order.  seq
+// numbers the reductions of a solve from 1.
 //
 // Each row's four lanes hold the terms of their component; two levels give the
 // row sums, lane v of a row then stores value v, and warp v adds the rows' v
 // sums: merging compensated pairs costs about nine instructions a level, so
 // the levels a full warp tree would run mostly on idle lanes are replaced by
 // one pass over shared memory.
-template <typename A, typename T, bool GRID>
+// ROWS: lane v of a row already holds the row's value v in a[0].
+template <typename A, typename T, bool GRID, bool ROWS = false>
 __device__ __forceinline__ void total3(A (&a)[3], ResShared<T>& sh, int k, int rank, unsigned seq, uint4* inbox) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (!ROWS)
 #pragma unroll
-  for (int v = 0; v < 3; ++v) {
-    a[v].shfl_merge(1);
-    a[v].shfl_merge(2);
-  }
+    for (int v = 0; v < 3; ++v) {
+      a[v].shfl_merge(1);
+      a[v].shfl_merge(2);
+    }
   if ((lane & 3) < 3) {
-    const A& m = (lane & 3) == 0 ? a[0] : (lane & 3) == 1 ? a[1] : a[2];
+    const A& m = ROWS || (lane & 3) == 0 ? a[0] : (lane & 3) == 1 ? a[1] : a[2];
     sh.red[lane & 3][warp * 8 + (lane >> 2)] = pack_word(m);
   }
   __syncthreads();
   const int par = seq & 1;
+  if (GRID && k > 1) {
+    // the sums go to kResCopies tables; a CTA polls the table of its rank
+    // (one table polled by 152 SMs: 4.8 us a reduction, its lines queue at
+    // their L2 slices; a table per CTA, 152^2 scattered sectors: 2.8 us)
+    const int pw = min(nw, 5), copies = min(k, kResCopies);
+    if (warp >= pw) return;
+    const unsigned np = 32u * (unsigned)pw;
+    if (warp < 3) {
+      A t;
+      for (int j = lane; j < nw * 8; j += 32) merge_word(t, sh.red[warp][j]);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) t.shfl_merge(o);
+      if (lane == 0) sh.tot[warp] = pack_word(t);
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(np) : "memory");
+    const u64 w0 = sh.tot[0], w1 = sh.tot[1], w2 = sh.tot[2];
+    const u64 h0 = (w2 & 0xffffffffull) | ((u64)seq << 32), h1 = (w2 >> 32) | ((u64)seq << 32);
+    for (int q = threadIdx.x; q < copies; q += (int)np) {
+      uint4* w = inbox + (((size_t)q * 2 + par) * k + rank) * 2;
+      st_word(w, w0, h0);
+      st_word(w + 1, w1, h1);
+    }
+    const int mine = rank % copies;
+    A g[3];
+    for (int i = threadIdx.x; i < k; i += (int)np) {
+      const uint4* w = inbox + (((size_t)mine * 2 + par) * k + i) * 2;
+      u64 x0, y0, x1, y1;
+      int tries = 0;
+      for (;;) {
+        ld_word(w, x0, y0);
+        ld_word(w + 1, x1, y1);
+        if (word_seq(y0) == seq && word_seq(y1) == seq) break;
+        if (++tries >= kResPollLimit) {
+          sh.abort_flag = 1;
+          break;
+        }
+      }
+      merge_word(g[0], x0);
+      merge_word(g[1], x1);
+      merge_word(g[2], (y0 & 0xffffffffull) | (y1 << 32));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+      for (int v = 0; v < 3; ++v) g[v].shfl_merge(o);
+    if (lane < 3) sh.part[lane][warp] = pack_word(lane == 0 ? g[0] : lane == 1 ? g[1] : g[2]);
+    asm volatile("bar.sync 1, %0;" ::"r"(np) : "memory");
+    if (warp == 0) {
+      A t;
+      const int v = lane >> 3, i = lane & 7;
+      if (v < 3 && i < pw) merge_word(t, sh.part[v][i]);
+      t.shfl_merge(1);
+      t.shfl_merge(2);
+      t.shfl_merge(4);
+      if (v < 3 && i == 0) sh.tot[v] = pack_word(t);
+      __syncwarp();
+    }
+    return;
+  }
   if (warp < 3) {
     A t;
     for (int j = lane; j < nw * 8; j += 32) merge_word(t, sh.red[warp][j]);
@@ -257,50 +367,27 @@ __device__ __forceinline__ void total3(A (&a)[3], ResShared<T>& sh, int k, int r
     const u64 w = pack_word(t);
     if (k == 1) {
       if (lane == 0) sh.tot[warp] = w;
-    } else if (GRID) {
-      // to every CTA's inbox; each polls its own, so no line is read by more
-      // than one SM (152 SMs polling the same lines queued at their L2
-      // slices: 4.8 us a reduction)
-      for (int q = lane; q < k; q += 32) st_word(inbox + (((size_t)q * 2 + par) * k + rank) * 3 + warp, w, (u64)seq << 32);
-      A g;
-      for (int i = lane; i < k; i += 32) {
-        u64 x, y;
-        int tries = 0;
-        for (;;) {
-          ld_word(inbox + (((size_t)rank * 2 + par) * k + i) * 3 + warp, x, y);
-          if (word_seq(y) == seq) break;
-          if (++tries >= kResPollLimit) {
-            sh.abort_flag = 1;
-            break;
-          }
-        }
-        merge_word(g, x);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) g.shfl_merge(o);
-      if (lane == 0) sh.tot[warp] = pack_word(g);
-    } else if (lane < k) {
-      st_async(cluster_map(smem_addr(&sh.slot[par][rank][warp]), lane), cluster_map(smem_addr(&sh.bar_s[par]), lane), w);
-    }
-    if (k == 1 || GRID) {
       asm volatile("bar.sync 1, 96;" ::: "memory");
-    } else if (warp == 0) {
-      if (!mbar_wait_cluster(&sh.bar_s[par], ((seq - 1) >> 1) & 1)) sh.abort_flag = 1;
-      __syncwarp();
-      if (lane == 0) mbar_expect_tx(&sh.bar_s[par], 24u * (unsigned)k);  // of its next use
-      // lane v * 8 + i adds the sums of CTAs i and i + 8
-      A g;
-      const int v = lane >> 3, i = lane & 7;
-      if (v < 3) {
-        if (i < k) merge_word(g, sh.slot[par][i][v]);
-        if (i + 8 < k) merge_word(g, sh.slot[par][i + 8][v]);
+    } else {
+      if (lane < k)
+        st_async(cluster_map(smem_addr(&sh.slot[par][rank][warp]), lane), cluster_map(smem_addr(&sh.bar_s[par]), lane), w);
+      if (warp == 0) {
+        if (!mbar_wait_cluster(&sh.bar_s[par], ((seq - 1) >> 1) & 1)) sh.abort_flag = 1;
+        __syncwarp();
+        // lane v * 8 + i adds the sums of CTAs i and i + 8
+        A g;
+        const int v = lane >> 3, i = lane & 7;
+        if (v < 3) {
+          if (i < k) merge_word(g, sh.slot[par][i][v]);
+          if (i + 8 < k) merge_word(g, sh.slot[par][i + 8][v]);
+        }
+        g.shfl_merge(1);
+        g.shfl_merge(2);
+        g.shfl_merge(4);
+        if (v < 3 && i == 0) sh.tot[v] = pack_word(g);
+        __syncwarp();
+        if (lane == 0) mbar_expect_tx(&sh.bar_s[par], 24u * (unsigned)k);  // of its next use
       }
-      g.shfl_merge(1);
-      g.shfl_merge(2);
-      g.shfl_merge(4);
-      if (v < 3 && i == 0) sh.tot[v] = pack_word(g);
-      __syncwarp();
     }
   }
 }
@@ -311,20 +398,28 @@ __device__ __forceinline__ void total3(A (&a)[3], ResShared<T>& sh, int k, int r
 // cycles here and its division 570: 2,200 cycles of every iteration), with
 // alpha = gamma / (delta - gamma (gamma / (gamma_old alpha_old))) so that no
 // squares leave FP32's range; alpha and beta are rounded to FP32 for the
-// update in both.
+// update in both.  The reciprocals of the old values are formed off the
+// critical path by scalars_next.
+__device__ __forceinline__ ff::dfloat word_ff(u64 w) {
+  return ff::fast_two_sum(__uint_as_float((unsigned)w), __uint_as_float((unsigned)(w >> 32)));
+}
+__device__ __forceinline__ u64 ff_word(ff::dfloat d) {
+  return (u64)__float_as_uint(d.hi) | ((u64)__float_as_uint(d.lo) << 32);
+}
 __device__ __forceinline__ void scalars(ResShared<float>& sh, int it, int max_it, double tol) {
   using namespace ff;
-  auto get = [](u64 w) { return fast_two_sum(__uint_as_float((unsigned)w), __uint_as_float((unsigned)(w >> 32))); };
-  auto put = [](dfloat d) { return (u64)__float_as_uint(d.hi) | ((u64)__float_as_uint(d.lo) << 32); };
-  const dfloat delta = get(sh.tot[0]), gamma = get(sh.tot[1]), rr = get(sh.tot[2]);
+  const dfloat delta = word_ff(sh.tot[0]), gamma = word_ff(sh.tot[1]), rr = word_ff(sh.tot[2]);
   if (it == 0) {
-    sh.rr0 = put(rr);
-    sh.thr = put(from_double(tol * tol * to_double(rr)));
+    sh.rr0 = ff_word(rr);
+    sh.thr = ff_word(from_double(tol * tol * to_double(rr)));
   }
-  const dfloat thr = get(sh.thr);
-  sh.rr = put(rr);
+  const dfloat thr = word_ff(sh.thr), iz = word_ff(sh.rz), iza = word_ff(sh.al);
+  dfloat alpha = make(0.f, 0.f), beta = make(0.f, 0.f), den = delta;
+  if (it > 0) {
+    beta = mul(gamma, iz);
+    den = sub(delta, mul(gamma, mul(gamma, iza)));
+  }
   int code = 0, fail = 0;
-  dfloat alpha = make(0.f, 0.f), beta = make(0.f, 0.f);
   if (sh.abort_flag) {
     code = 2;
     fail = 5;
@@ -335,26 +430,26 @@ __device__ __forceinline__ void scalars(ResShared<float>& sh, int it, int max_it
     code = 1;
   } else if (it >= max_it) {
     code = 3;
+  } else if (!(den.hi > 0.f) || !isfinite(den.hi)) {
+    code = 2;
+    fail = isfinite(den.hi) ? 2 : 3;
   } else {
-    dfloat den = delta;
-    if (it > 0) {
-      const dfloat rz = get(sh.rz);
-      beta = mul(gamma, rcp(rz));
-      den = sub(delta, mul(gamma, mul(beta, rcp(get(sh.al)))));
-    }
-    if (!(den.hi > 0.f) || !isfinite(den.hi)) {
-      code = 2;
-      fail = isfinite(den.hi) ? 2 : 3;
-    } else {
-      alpha = mul(gamma, rcp(den));
-    }
+    alpha = mul(gamma, rcp(den));
   }
-  sh.rz = put(gamma);
-  sh.al = put(alpha);
   sh.coef[0] = alpha.hi;
   sh.coef[1] = beta.hi;
   sh.code = code;
   sh.fail = fail;
+  sh.rr = ff_word(rr);
+  sh.tot[0] = ff_word(alpha);  // for scalars_next
+}
+// 1 / gamma and 1 / (gamma alpha) for the next iteration (one thread, after
+// the barrier that publishes alpha and beta)
+__device__ __forceinline__ void scalars_next(ResShared<float>& sh) {
+  using namespace ff;
+  const dfloat iz = rcp(word_ff(sh.tot[1]));
+  sh.rz = ff_word(iz);
+  sh.al = ff_word(mul(iz, rcp(word_ff(sh.tot[0]))));
 }
 __device__ __forceinline__ void scalars(ResShared<double>& sh, int it, int max_it, double tol) {
   auto get = [](u64 w) { return __longlong_as_double((long long)w); };
@@ -399,6 +494,7 @@ __device__ __forceinline__ void scalars(ResShared<double>& sh, int it, int max_i
   sh.code = code;
   sh.fail = fail;
 }
+__device__ __forceinline__ void scalars_next(ResShared<double>&) {}
 __device__ __forceinline__ double word_value(const ResShared<float>&, u64 w) {
   return (double)__uint_as_float((unsigned)w) + (double)__uint_as_float((unsigned)(w >> 32));
 }
@@ -454,43 +550,59 @@ template <typename T, bool GRID, bool BLK>
 __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResItem& I, int item, int rank,
                                                unsigned char* smem, ResShared<T>& sh) {
   using V = typename Vec4<T>::type;
-  constexpr int NS = ResShape<T>::slots, RB = ResShape<T>::reg, RA = RB > 0 ? RB : 1, NM = BLK ? 3 : 1;
+  using Shape = ResShape<T>;
+  constexpr bool F32 = sizeof(T) == 4;
+  constexpr int NS = Shape::slots, RB = Shape::reg, OFF = Shape::off, RA = RB > 0 ? RB : 1, NM = BLK ? 3 : 1;
   const ResPlanDev P = A.plans[I.plan];
   const int k = P.k;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, c = lane & 3, q0 = lane & ~3;
   const int ch0 = P.part_chunk[rank], nch = P.part_chunk[rank + 1] - ch0;
   const int4 win = P.part_win[rank];
   const int row0 = ch0 * kResChunkRows, row1 = min(P.rows, (ch0 + nch) * kResChunkRows);
-  // shared memory: the window [columns][4], the values that are not in
-  // registers [steps][9][32], the column indices of every step [steps][32]
+  // shared memory: the window [columns][4]; FP32: every chunk's p, s, x and
+  // preconditioner [chunks][.][32]; the values that are in neither registers
+  // nor tensor memory [steps][9][32]; the columns of every step [steps][32]
   V* uw = reinterpret_cast<V*>(smem);
-  const int steps0 = P.chunk_step[ch0], allsteps = P.chunk_step[ch0 + nch] - steps0;
+  const int steps0 = P.chunk_step[ch0];
   int vstep[NS], cstep[NS], nst[NS];  // first value step, first index step, steps of this warp's chunks
   int vsteps = 0;                     // value steps in shared memory
   {
-    // the first nw chunks keep RB steps in registers
-    int pre = 0, mine = 0;
-    for (int i = 0; i < min(nw, nch); ++i) {
-      if (i == warp) mine = pre;
-      pre += max(0, P.chunk_step[ch0 + i + 1] - P.chunk_step[ch0 + i] - RB);
-    }
-    const int first = nch > nw ? P.chunk_step[ch0 + nw] : P.chunk_step[ch0 + nch];
 #pragma unroll
-    for (int q = 0; q < NS; ++q) {
-      const int i = warp + q * nw;
-      const bool on = i < nch;
-      const int s0 = on ? P.chunk_step[ch0 + i] : 0;
-      nst[q] = on ? P.chunk_step[ch0 + i + 1] - s0 : 0;
-      cstep[q] = on ? s0 - steps0 : 0;
-      vstep[q] = q == 0 ? mine : (on ? pre + s0 - first : 0);
+    for (int q = 0; q < NS; ++q) vstep[q] = cstep[q] = nst[q] = 0;
+    for (int i0 = 0; i0 < nch; i0 += 32) {
+      const int i = i0 + lane;
+      const int b = i < nch ? P.chunk_step[ch0 + i] : 0, n = i < nch ? P.chunk_step[ch0 + i + 1] - b : 0;
+      const int v = i < OFF * nw ? max(0, n - RB) : n;
+      int inc = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+      }
+#pragma unroll
+      for (int q = 0; q < NS; ++q) {
+        const int mine = warp + q * nw;  // this warp's chunk of slot q
+        const int from = mine & 31;
+        const int ve = __shfl_sync(0xffffffffu, vsteps + inc - v, from), ce = __shfl_sync(0xffffffffu, b, from),
+                  ne = __shfl_sync(0xffffffffu, n, from);
+        if (mine < nch && mine >= i0 && mine < i0 + 32) {
+          vstep[q] = ve;
+          cstep[q] = ce - steps0;
+          nst[q] = ne;
+        }
+      }
+      vsteps += __shfl_sync(0xffffffffu, inc, 31);
     }
-    vsteps = pre + (steps0 + allsteps - first);
   }
-  T* vals = reinterpret_cast<T*>(uw + win.y);
+  T* state = reinterpret_cast<T*>(uw + win.y);  // p, s, x
+  T* prec = state + (F32 ? (size_t)nch * 3 * 32 : 0);
+  T* vals = prec + (F32 ? (size_t)nch * NM * 32 : 0);
   uint16_t* cols = reinterpret_cast<uint16_t*>(vals + (size_t)vsteps * 9 * 32);
   uint4* inbox = GRID ? A.ll + I.ll : nullptr;                         // partial sums
-  uint4* urow = GRID ? inbox + 6 * (size_t)k * k : nullptr;            // rows' vectors
-  for (int i = threadIdx.x; i < 3 * 128; i += blockDim.x) (&sh.red[0][0])[i] = 0;
+  uint4* urow = GRID ? inbox + 4 * (size_t)min(k, kResCopies) * k : nullptr;  // rows' vectors
+  // columns of this warp's quarter: two chunks of 64
+  const unsigned tm = F32 ? sh.tmem + ((unsigned)(warp & 3) << 21) + (unsigned)(warp >> 2) * 128u : 0u;
+  const long long at0 = (long long)I.vec * A.nnd + I.node_off;  // of this right-hand side
   if (threadIdx.x == 0) sh.abort_flag = 0;
   if (!GRID && k > 1) {
     if (threadIdx.x < k) {
@@ -512,23 +624,31 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
   }
   // --- the rows of the part, assembled from the element blocks
   T rv[RA][9];
-  T Mi[NS][NM];
-  unsigned comp = 0;  // bit q: this lane's component of its row in chunk q is a free dof
-  bool live[NS];
+  T Mr[NS][NM], pr[NS], sr[NS], xr[NS];  // registers in FP64; FP32 keeps them in shared memory
+  unsigned comp = 0;   // bit q: this lane's component of its row in chunk q is a free dof
+  unsigned live = 0;   // bit q: the row exists
+  unsigned peers[NS];  // cluster form: the other parts whose windows hold the row
 #pragma unroll
   for (int q = 0; q < NS; ++q) {
-    const int row = (ch0 + warp + q * nw) * kResChunkRows + (lane >> 2);
-    live[q] = nst[q] > 0 && row < P.rows;
-    const uint8_t m = live[q] ? A.mask[I.node_off + P.act_node[row]] : 0;
+    const int i = warp + q * nw;
+    const int row = (ch0 + i) * kResChunkRows + (lane >> 2);
+    const bool lv = i < nch && row < P.rows;
+    if (lv) live |= 1u << q;
+    const uint8_t m = lv ? A.mask[I.node_off + P.act_node[row]] : 0;
     if (c < 3 && ((m >> c) & 1)) comp |= 1u << q;
+    peers[q] = 0u;
+    if (!GRID && k > 1 && lv && c == 0)
+      for (int o = win.z; o <= win.w; ++o)
+        if (o != rank && row >= sh.peer[o].x && row < sh.peer[o].x + sh.peer[o].y) peers[q] |= 1u << o;
     T D[9];
     bool have = false;
     auto block = [&](int t, T acc[9]) {
-      const int i = (steps0 + cstep[q] + t) * 32 + lane;
-      const int cl = P.col[i];
-      slot_value<T>(P.slot[i], m, P.contrib, A.Ke, I.elem_off, acc);
+      const int at = (steps0 + cstep[q] + t) * 32 + lane;
+      const int cl = P.col[at];
+      const int2 sl = P.slot[at];
+      slot_value<T>(sl, m, P.contrib, A.Ke, I.elem_off, acc);
       cols[(size_t)(cstep[q] + t) * 32 + lane] = (uint16_t)(cl - win.x);
-      if (cl == row && P.slot[i].y > 0) {
+      if (cl == row && sl.y > 0) {
         have = true;
 #pragma unroll
         for (int e = 0; e < 9; ++e) D[e] = acc[e];
@@ -547,10 +667,19 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
         }
       }
     }
-    for (int t = q == 0 ? RB : 0; t < nst[q]; ++t) {
+    if constexpr (F32) {
+      if (q > 0 && q < OFF)
+        for (int t = 0; t < min(RB, nst[q]); ++t) {
+          T acc[9];
+          block(t, acc);
+          __syncwarp();
+          tmem_st9(tm + (unsigned)(q - 1) * 64u + 9u * (unsigned)t, acc);
+        }
+    }
+    for (int t = q < OFF ? RB : 0; t < nst[q]; ++t) {
       T acc[9];
       block(t, acc);
-      T* vp = vals + (size_t)(vstep[q] + t - (q == 0 ? RB : 0)) * 9 * 32 + lane;
+      T* vp = vals + (size_t)(vstep[q] + t - (q < OFF ? RB : 0)) * 9 * 32 + lane;
 #pragma unroll
       for (int e = 0; e < 9; ++e) vp[32 * e] = acc[e];
     }
@@ -563,22 +692,42 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
     diagonal_inverses<T>(m, D, Dg, B);
 #pragma unroll
     for (int d = 0; d < NM; ++d) {
-      if (BLK)
-        Mi[q][d] = c == 0 ? B[d] : c == 1 ? B[3 + d] : c == 2 ? B[6 + d] : T(0);
-      else
-        Mi[q][d] = c == 0 ? Dg[0] : c == 1 ? Dg[4] : c == 2 ? Dg[8] : T(0);
-      if (!who || !live[q]) Mi[q][d] = T(0);
+      T v = BLK ? (c == 0 ? B[d] : c == 1 ? B[3 + d] : c == 2 ? B[6 + d] : T(0))
+                : (c == 0 ? Dg[0] : c == 1 ? Dg[4] : c == 2 ? Dg[8] : T(0));
+      if (!who || !lv) v = T(0);
+      if (F32) {
+        if (i < nch) prec[((size_t)i * NM + d) * 32 + lane] = v;
+      } else {
+        Mr[q][d] = v;
+      }
+    }
+    if (F32) {
+      if (i < nch)
+#pragma unroll
+        for (int v = 0; v < 3; ++v) state[((size_t)i * 3 + v) * 32 + lane] = T(0);
+    } else {
+      pr[q] = sr[q] = xr[q] = T(0);
     }
   }
+  if constexpr (F32) tmem_wait_st();
+  // M^-1 r of a row's component (whole warps; zero for a warp without a chunk)
   auto precond = [&](int q, T rq) {
-    if (!BLK) return Mi[q][0] * rq;
+    const bool on = warp + q * nw < nch;
+    const T* Mq = prec + (size_t)(on ? warp + q * nw : 0) * NM * 32 + lane;
     T z = T(0);
 #pragma unroll
-    for (int d = 0; d < NM; ++d) z += Mi[q][d] * __shfl_sync(0xffffffffu, rq, q0 + d);
+    for (int d = 0; d < NM; ++d) {
+      T m;
+      if constexpr (F32)
+        m = on ? Mq[32 * d] : T(0);
+      else
+        m = Mr[q][d];
+      z += m * (BLK ? __shfl_sync(0xffffffffu, rq, q0 + d) : rq);
+    }
     return z;
   };
   unsigned seq = 0;
-  T r[NS], p[NS], s[NS], x[NS], u[NS];
+  T r[NS], u[NS];
   int scale_exp = 0;
   {
     // --- the right-hand side on a power of two near its size: first by its
@@ -589,7 +738,7 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
       const int row = (ch0 + warp + q * nw) * kResChunkRows + (lane >> 2);
-      b[q] = ((comp >> q) & 1) ? reinterpret_cast<const double*>(A.rhs + (I.node_off + P.act_node[row]))[c] : 0.0;
+      b[q] = ((comp >> q) & 1) ? reinterpret_cast<const double*>(A.rhs + (at0 + P.act_node[row]))[c] : 0.0;
       a[0].v = max(a[0].v, exponent_of(b[q]));
     }
     ++seq;
@@ -601,6 +750,7 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
     a[0].v = a[1].v = a[2].v = 0;
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
+      if (q * nw >= nch) break;
       const T rq = T(b[q] * sc);
       a[0].v = max(a[0].v, exponent_of((double)(rq * precond(q, rq))));
     }
@@ -614,8 +764,8 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
       r[q] = T(b[q] * sc);
-      p[q] = s[q] = x[q] = T(0);
-      u[q] = precond(q, r[q]);
+      u[q] = T(0);
+      if (q * nw < nch) u[q] = precond(q, r[q]);
     }
     __syncthreads();
   }
@@ -627,24 +777,33 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
     for (int q = 0; q < NS; ++q) {
       if (q * nw >= nch) break;
       const T u1 = __shfl_down_sync(0xffffffffu, u[q], 1), u2 = __shfl_down_sync(0xffffffffu, u[q], 2);
-      if (live[q] && c == 0) {
+      if (((live >> q) & 1) && c == 0) {
         const int row = (ch0 + warp + q * nw) * kResChunkRows + (lane >> 2);
         uw[row - win.x] = mk<V, T>(u[q], u1, u2);
-        if (k > 1) {
-          if (GRID) {
-            RowWords<T>::store(urow + (size_t)row * RowWords<T>::n, u[q], u1, u2, (unsigned)it + 1u);
-          } else {
-            for (int o = win.z; o <= win.w; ++o) {
-              if (o == rank) continue;
-              const int4 pq = sh.peer[o];
-              const int at = row - pq.x;
-              if (at >= 0 && at < pq.y)
-                st_async_row((unsigned)pq.z + (unsigned)(at * (int)sizeof(V)), (unsigned)pq.w, u[q], u1, u2);
-            }
-          }
+        if (GRID && k > 1) RowWords<T>::store(urow + (size_t)row * RowWords<T>::n, u[q], u1, u2, (unsigned)it + 1u);
+        for (unsigned to = peers[q]; to; to &= to - 1) {
+          const int4 pq = sh.peer[__ffs((int)to) - 1];
+          st_async_row((unsigned)pq.z + (unsigned)((row - pq.x) * (int)sizeof(V)), (unsigned)pq.w, u[q], u1, u2);
         }
       }
     }
+    __syncwarp();
+    if (!GRID && k > 1 && lane == 0) {
+      if (warp == 0)
+        mbar_expect_tx(&sh.bar_u, (unsigned)((win.y - (row1 - row0)) * (int)sizeof(V)));
+      else
+        mbar_arrive(&sh.bar_u);
+    }
+    if (warp == 1 && lane == 0 && it > 0) scalars_next(sh);
+    // gamma and r.r while the vectors travel
+    Acc<T> a[3];
+    if (F32)
+#pragma unroll
+      for (int q = 0; q < NS; ++q)
+        if ((comp >> q) & 1) {
+          a[1].add_prod(r[q], u[q]);
+          a[2].add_prod(r[q], r[q]);
+        }
     __syncwarp();
     if (GRID && k > 1) {
       // the other parts' rows of the window: below and above this part's
@@ -663,23 +822,16 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
       }
       __syncthreads();
     } else if (!GRID && k > 1) {
-      if (lane == 0) {
-        if (warp == 0)
-          mbar_expect_tx(&sh.bar_u, (unsigned)((win.y - (row1 - row0)) * (int)sizeof(V)));
-        else
-          mbar_arrive(&sh.bar_u);
-      }
       if (!mbar_wait_cluster(&sh.bar_u, (unsigned)it & 1u)) sh.abort_flag = 1;
       __syncwarp();
     } else {
       __syncthreads();
     }
-    // w = A u, one chunk after the other; component c of a row on its lane c
-    T w[NS];
-    Acc<T> a[3];
+    // w = A u, one chunk after the other
+    T w[NS], A0[NS], A1[NS], A2[NS];
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
-      w[q] = T(0);
+      A0[q] = A1[q] = A2[q] = T(0);
       if (q * nw >= nch) break;
       T a0 = T(0), a1 = T(0), a2 = T(0);
       const uint16_t* cp = cols + (size_t)cstep[q] * 32 + lane;
@@ -692,32 +844,74 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
             a1 += rv[t][3] * uj.x + rv[t][4] * uj.y + rv[t][5] * uj.z;
             a2 += rv[t][6] * uj.x + rv[t][7] * uj.y + rv[t][8] * uj.z;
           }
-        cp += 32 * RB;
       }
+      if constexpr (F32) {
+        if (q > 0 && q < OFF) {
+          const unsigned col = tm + (unsigned)(q - 1) * 64u;
+          auto step = [&](int t, const unsigned* b) {
+            const V uj = uw[cp[32 * t]];
+            a0 += __uint_as_float(b[0]) * uj.x + __uint_as_float(b[1]) * uj.y + __uint_as_float(b[2]) * uj.z;
+            a1 += __uint_as_float(b[3]) * uj.x + __uint_as_float(b[4]) * uj.y + __uint_as_float(b[5]) * uj.z;
+            a2 += __uint_as_float(b[6]) * uj.x + __uint_as_float(b[7]) * uj.y + __uint_as_float(b[8]) * uj.z;
+          };
+#pragma unroll
+          for (int t = 0; t < RB; t += 2)
+            if (t < nst[q]) {
+              unsigned b[18];
+              __syncwarp();
+              if (t + 1 < RB)
+                tmem_ld18(col + 9u * (unsigned)t, b);
+              else
+                tmem_ld9(col + 9u * (unsigned)t, b);
+              tmem_wait_ld();
+              step(t, b);
+              if (t + 1 < RB && t + 1 < nst[q]) step(t + 1, b + 9);
+            }
+        }
+      }
+      const int t0 = q < OFF ? RB : 0;
+      cp += 32 * t0;
       const T* vp = vals + (size_t)vstep[q] * 9 * 32 + lane;
 #pragma unroll 4
-      for (int t = q == 0 ? RB : 0; t < nst[q]; ++t, vp += 9 * 32, cp += 32) {
+      for (int t = t0; t < nst[q]; ++t, vp += 9 * 32, cp += 32) {
         const V uj = uw[*cp];
         a0 += vp[0] * uj.x + vp[32] * uj.y + vp[64] * uj.z;
         a1 += vp[96] * uj.x + vp[128] * uj.y + vp[160] * uj.z;
         a2 += vp[192] * uj.x + vp[224] * uj.y + vp[256] * uj.z;
       }
-      // lanes 0, 1 of a row keep components 0 and 1, lanes 2, 3 component 2
+      A0[q] = a0;
+      A1[q] = a1;
+      A2[q] = a2;
+    }
+    // sums over a row's lanes, component c to lane c: lanes 0, 1 keep
+    // components 0 and 1, lanes 2, 3 component 2
+#pragma unroll
+    for (int q = 0; q < NS; ++q) {
+      w[q] = T(0);
+      if (q * nw >= nch) break;
       const bool up = (c & 2) != 0;
-      const T g0 = __shfl_xor_sync(0xffffffffu, up ? a0 : a2, 2);
-      const T g1 = __shfl_xor_sync(0xffffffffu, a1, 2);
-      const T b0 = (up ? a2 : a0) + g0;
-      const T b1 = a1 + g1;
+      const T g0 = __shfl_xor_sync(0xffffffffu, up ? A0[q] : A2[q], 2);
+      const T g1 = __shfl_xor_sync(0xffffffffu, A1[q], 2);
+      const T b0 = (up ? A2[q] : A0[q]) + g0;
+      const T b1 = A1[q] + g1;
       const T e = __shfl_xor_sync(0xffffffffu, up ? b0 : ((c & 1) ? b0 : b1), 1);
       w[q] = up ? b0 + e : ((c & 1) ? b1 + e : b0 + e);
-      if ((comp >> q) & 1) {
-        a[0].add_prod(u[q], w[q]);
-        a[1].add_prod(r[q], u[q]);
-        a[2].add_prod(r[q], r[q]);
+      if (F32) {
+        if ((comp >> q) & 1) a[0].add_prod(u[q], w[q]);
+      } else {
+        // lane v of a row forms the row's value v from its gathered
+        // components: three FP64 operations where the lanes' own terms and
+        // their two merging levels took nine
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const T ud = __shfl_sync(0xffffffffu, u[q], q0 + d), rd = __shfl_sync(0xffffffffu, r[q], q0 + d),
+                  wd = __shfl_sync(0xffffffffu, w[q], q0 + d);
+          a[0].add_prod(c == 2 ? rd : ud, c == 0 ? wd : rd);
+        }
       }
     }
     ++seq;
-    total3<Acc<T>, T, GRID>(a, sh, k, rank, seq, inbox);
+    total3<Acc<T>, T, GRID, !F32>(a, sh, k, rank, seq, inbox);
     if (threadIdx.x == 0) scalars(sh, it, A.max_it, A.tol);
     __syncthreads();
     if (sh.code) break;
@@ -725,10 +919,22 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
       if (q * nw >= nch) break;
-      p[q] = u[q] + be * p[q];
-      s[q] = w[q] + be * s[q];
-      x[q] += al * p[q];
-      r[q] -= al * s[q];
+      if (F32) {
+        T* sq = state + (size_t)(warp + q * nw) * 3 * 32 + lane;
+        if (warp + q * nw < nch) {
+          const T pn = u[q] + be * sq[0], sn = w[q] + be * sq[32];
+          sq[64] += al * pn;
+          sq[0] = pn;
+          sq[32] = sn;
+          r[q] -= al * sn;
+        }
+      } else {
+        pr[q] = u[q] + be * pr[q];
+        sr[q] = w[q] + be * sr[q];
+        xr[q] += al * pr[q];
+        r[q] -= al * sr[q];
+      }
+      __syncwarp();
       u[q] = precond(q, r[q]);
     }
   }
@@ -736,11 +942,13 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
   const int code = sh.code;
 #pragma unroll
   for (int q = 0; q < NS; ++q) {
-    T xq = x[q];
+    if (q * nw >= nch) break;
+    const int i = warp + q * nw;
+    T xq = F32 ? (i < nch ? state[((size_t)i * 3 + 2) * 32 + lane] : T(0)) : xr[q];
     if (A.batch) xq = code == 2 ? T(0) : xq * T(unscale);
     const T x1 = __shfl_down_sync(0xffffffffu, xq, 1), x2 = __shfl_down_sync(0xffffffffu, xq, 2);
-    const int row = (ch0 + warp + q * nw) * kResChunkRows + (lane >> 2);
-    if (live[q] && c == 0) A.x[I.node_off + P.act_node[row]] = mk<V, T>(xq, x1, x2);
+    const int row = (ch0 + i) * kResChunkRows + (lane >> 2);
+    if (((live >> q) & 1) && c == 0) A.x[at0 + P.act_node[row]] = mk<V, T>(xq, x1, x2);
   }
   if (threadIdx.x == 0) {
     if (sh.fail == 5) atomicOr(A.status, kStatusWaitTimeout);
@@ -766,24 +974,109 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
   }
 }
 
+// Tensor memory of a CTA with all its warps: such a CTA has the SM to itself
+// (512 threads at 128 registers), so the allocation never waits for another.
+template <typename T>
+__device__ __forceinline__ bool tmem_begin(ResShared<T>& sh) {
+  const bool use = sizeof(T) == 4 && blockDim.x == ResShape<T>::warps * 32;
+  if (use && threadIdx.x < 32) tmem_alloc(&sh.tmem);
+  __syncthreads();
+  return use;
+}
+template <typename T>
+__device__ __forceinline__ void tmem_end(ResShared<T>& sh, bool use) {
+  __syncthreads();
+  if (use && threadIdx.x < 32) tmem_free(sh.tmem);
+}
+
 template <typename T, bool BLK>
 __global__ void __launch_bounds__(ResShape<T>::warps * 32, 1) resident_cluster_kernel(ResArgs<T> A) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ ResShared<T> sh;
   const int item = blockIdx.x / A.k, rank = blockIdx.x % A.k;
+  const bool tmem = tmem_begin(sh);
   resident_solve<T, false, BLK>(A, A.items[item], item, rank, smem, sh);
+  tmem_end(sh, tmem);
 }
 
 template <typename T, bool BLK>
 __global__ void __launch_bounds__(ResShape<T>::warps * 32, 1) resident_grid_kernel(ResArgs<T> A) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ ResShared<T> sh;
+  const bool tmem = tmem_begin(sh);
   for (int e = A.sched_ptr[blockIdx.x]; e < A.sched_ptr[blockIdx.x + 1]; ++e) {
     const int2 w = A.sched[e];
     resident_solve<T, true, BLK>(A, A.items[w.x], w.x, w.y, smem, sh);
     const bool stop = sh.abort_flag != 0;
     __syncthreads();
-    if (stop) return;  // a wait ran out: nothing more is awaited
+    if (stop) break;  // a wait ran out: nothing more is awaited
+  }
+  tmem_end(sh, tmem);
+}
+
+// The rows of a whole mesh on the device (a mesh of 50,000 nodes took 17 ms on
+// the host, as long as its load step).  rank: index of every active node.
+__global__ void rows_flag_kernel(int n, const uint8_t* __restrict__ mask, int* __restrict__ flag) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) flag[i] = mask[i] ? 1 : 0;
+}
+__global__ void rows_node_kernel(int n, const uint8_t* __restrict__ mask, const int* __restrict__ rank,
+                                 int* __restrict__ act_node) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n && mask[i]) act_node[rank[i]] = i;
+}
+// one warp per chunk, four lanes per row: steps and column range (FILL
+// false), or the blocks and columns of every step (FILL true); a row's active
+// blocks go to its lanes in turn
+template <bool FILL>
+__global__ void __launch_bounds__(256) rows_chunk_kernel(int rows, int nch, const int* __restrict__ act_node,
+                                                         const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                         const uint8_t* __restrict__ mask,
+                                                         const int* __restrict__ rank, int* __restrict__ step,
+                                                         int* __restrict__ lo, int* __restrict__ hi,
+                                                         int* __restrict__ blk, int* __restrict__ cidx) {
+  const int ch = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, c = lane & 3;
+  if (ch >= nch) return;
+  const int r0 = ch * kResChunkRows, row = r0 + (lane >> 2);
+  const bool live = row < rows;
+  const int g = live ? act_node[row] : 0;
+  const int b = live ? rowptr[g] : 0, e = live ? rowptr[g + 1] : 0;
+  int l = r0, h = min(rows, r0 + kResChunkRows), cnt = 0;
+  const int s0 = FILL ? step[ch] : 0, s1 = FILL ? step[ch + 1] : 0;
+  if (FILL)
+    for (int t = s0; t < s1; ++t) {
+      blk[(size_t)t * 32 + lane] = -1;
+      cidx[(size_t)t * 32 + lane] = r0;
+    }
+  __syncwarp();
+  for (int j0 = b; __any_sync(0xffffffffu, j0 < e); j0 += 4) {
+    const int j = j0 + c;
+    const bool on = j < e && mask[col[j]] != 0;
+    const unsigned m = (__ballot_sync(0xffffffffu, on) >> (lane & ~3)) & 0xfu;
+    if (on) {
+      const int a = rank[col[j]], q = cnt + __popc(m & ((1u << c) - 1u));
+      l = min(l, a);
+      h = max(h, a + 1);
+      if (FILL) {
+        const size_t at = (size_t)(s0 + (q >> 2)) * 32 + (lane & ~3) + (q & 3);
+        blk[at] = j;
+        cidx[at] = a;
+      }
+    }
+    cnt += __popc(m);
+  }
+  if (!FILL) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      l = min(l, __shfl_xor_sync(0xffffffffu, l, o));
+      h = max(h, __shfl_xor_sync(0xffffffffu, h, o));
+      cnt = max(cnt, __shfl_xor_sync(0xffffffffu, cnt, o));
+    }
+    if (lane == 0) {
+      step[ch] = (cnt + 3) / 4;
+      lo[ch] = l;
+      hi[ch] = h;
+    }
   }
 }
 
@@ -861,7 +1154,7 @@ void resident_rows(int n0, int n1, const int* rowptr, const int* col, const uint
       id[i] = (int)R.act_node.size();
       R.act_node.push_back(i);
     }
-  const int rows = (int)R.act_node.size(), nch = (rows + kResChunkRows - 1) / kResChunkRows;
+  const int rows = R.rows = (int)R.act_node.size(), nch = (rows + kResChunkRows - 1) / kResChunkRows;
   R.chunk_step.assign(nch + 1, 0);
   R.chunk_lo.assign(nch, 0);
   R.chunk_hi.assign(nch, 0);
@@ -903,24 +1196,25 @@ void resident_rows(int n0, int n1, const int* rowptr, const int* col, const uint
 
 namespace {
 
-// Bytes of one part with nw warps: the window, the values outside registers
-// (the first nw chunks keep `reg` steps there), the columns of every step.
-size_t part_bytes(const ResRows& R, int a, int b, int elem, int reg, int nw, int* lo, int* hi) {
+// Bytes of one part with nw warps: the window, FP32's vectors and
+// preconditioner, the values outside registers and tensor memory (the first
+// off * nw chunks keep `reg` steps there), the columns of every step.
+size_t part_bytes(const ResRows& R, int a, int b, int elem, int reg, int off, int state, int nw, int* lo, int* hi) {
   int l = R.chunk_lo[a], h = R.chunk_hi[a];
   size_t vsteps = 0;
   for (int ch = a; ch < b; ++ch) {
     l = std::min(l, R.chunk_lo[ch]);
     h = std::max(h, R.chunk_hi[ch]);
     const int n = R.chunk_step[ch + 1] - R.chunk_step[ch];
-    vsteps += ch - a < nw ? std::max(0, n - reg) : n;
+    vsteps += ch - a < off * nw ? std::max(0, n - reg) : n;
   }
   *lo = l;
   *hi = h;
   const size_t steps = (size_t)(R.chunk_step[b] - R.chunk_step[a]);
-  return (size_t)(h - l) * 4 * elem + vsteps * 9 * 32 * elem + steps * 64;
+  return (size_t)(h - l) * 4 * elem + (size_t)(b - a) * state * 32 * elem + vsteps * 9 * 32 * elem + steps * 64;
 }
 
-// The chunks cut into k consecutive parts of near-equal steps; false if one
+// The chunks cut into k consecutive parts of near-equal work; false if one
 // exceeds a CTA.
 bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
   const int nch = (int)R.chunk_lo.size();
@@ -928,13 +1222,25 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
   const int warps = elem == 4 ? ResShape<float>::warps : ResShape<double>::warps;
   const int slots = elem == 4 ? ResShape<float>::slots : ResShape<double>::slots;
   const int reg = elem == 4 ? ResShape<float>::reg : ResShape<double>::reg;
-  const long long total = R.chunk_step[nch];
+  const int off = elem == 4 ? ResShape<float>::off : ResShape<double>::off;
+  const int state = elem == 4 ? ResShape<float>::state : ResShape<double>::state;
+  // a chunk's work is its steps and its vector updates (about two steps')
+  auto work = [&](int ch) { return (long long)R.chunk_step[ch] + 2LL * ch; };
+  const long long total = work(nch);
   P.part_chunk.assign(k + 1, 0);
   P.part_chunk[k] = nch;
   for (int q = 1; q < k; ++q) {
     const long long target = (total * q + k / 2) / k;
-    int ch = (int)(std::lower_bound(R.chunk_step.begin(), R.chunk_step.end(), (int)target) - R.chunk_step.begin());
-    if (ch > 0 && target - R.chunk_step[ch - 1] < R.chunk_step[ch] - target) --ch;
+    int lo = 0, hi = nch;  // first chunk start with at least the target before it
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (work(mid) < target)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    int ch = lo;
+    if (ch > 0 && target - work(ch - 1) < work(ch) - target) --ch;
     P.part_chunk[q] = std::min(std::max(ch, P.part_chunk[q - 1] + 1), nch - (k - q));
   }
   P.part_win.assign(k, make_int4(0, 0, 0, 0));
@@ -947,7 +1253,7 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
   for (int q = 0; q < k; ++q) {
     const int a = P.part_chunk[q], b = P.part_chunk[q + 1];
     int lo, hi;
-    const size_t bytes = part_bytes(R, a, b, elem, reg, P.warps, &lo, &hi);
+    const size_t bytes = part_bytes(R, a, b, elem, reg, off, state, P.warps, &lo, &hi);
     if (bytes > cap || hi - lo > 65535) return false;
     P.smem = std::max(P.smem, bytes);
     P.part_win[q] = make_int4(lo, hi - lo, q, q);
@@ -973,7 +1279,7 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
 // (grid) CTAs of a cooperative launch.
 bool resident_plan(const ResRows& R, int elem, int num_sms, size_t cap, int max_cluster, bool alone, ResPlan& P) {
   const int nch = (int)R.chunk_lo.size();
-  P.rows = (int)R.act_node.size();
+  P.rows = R.rows;
   P.nchunks = nch;
   if (nch == 0) return false;
   const int most = elem == 4 ? ResShape<float>::warps * ResShape<float>::slots
@@ -1043,6 +1349,64 @@ int resident_slots(Context* c, long long n, const int* d_blk, const int* d_cptr,
   return ok(c, cudaGetLastError(), "resident_slots_kernel") ? TG_OK : TG_ERR_CUDA;
 }
 
+namespace {
+// Rows of the whole mesh on the device; R receives what the split needs.
+int rows_of_mesh(Context* c, ResRows& R, ResPlanDev& D) {
+  R = ResRows{};
+  const int n = c->nnd;
+  cudaStream_t st = c->stream;
+  int *flag = nullptr, *rank = nullptr, *tmp = nullptr, *node = nullptr;
+  if (!dalloc(c, &flag, (size_t)n) || !dalloc(c, &rank, (size_t)n + 1) || !dalloc(c, &tmp, (size_t)n / 1024 + 4))
+    return TG_ERR_OOM;
+  rows_flag_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, c->d_mask, flag);
+  int s = scan_counts(c, n, flag, rank, tmp);
+  if (s) return s;
+  if (!ok(c, cudaMemcpyAsync(&R.rows, rank + n, sizeof(int), cudaMemcpyDeviceToHost, st), "rows") ||
+      !ok(c, cudaStreamSynchronize(st), "sync"))
+    return TG_ERR_CUDA;
+  const int nch = (R.rows + kResChunkRows - 1) / kResChunkRows;
+  R.chunk_step.assign(nch + 1, 0);
+  R.chunk_lo.assign(nch, 0);
+  R.chunk_hi.assign(nch, 0);
+  c->launches++;
+  if (nch == 0) return TG_OK;
+  int *cnt = nullptr, *step = nullptr, *lohi = nullptr;
+  if (!dalloc(c, &node, (size_t)R.rows) || !dalloc(c, &cnt, (size_t)nch) || !dalloc(c, &step, (size_t)nch + 1) ||
+      !dalloc(c, &lohi, 2 * (size_t)nch))
+    return TG_ERR_OOM;
+  rows_node_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, c->d_mask, rank, node);
+  const int grid = (nch + 7) / 8;
+  rows_chunk_kernel<false><<<grid, 256, 0, st>>>(R.rows, nch, node, c->d_rowptr, c->d_col, c->d_mask, rank, cnt, lohi,
+                                                 lohi + nch, nullptr, nullptr);
+  s = scan_counts(c, nch, cnt, step, tmp);
+  if (s) return s;
+  if (!ok(c, cudaGetLastError(), "rows kernels") ||
+      !ok(c, cudaMemcpyAsync(R.chunk_step.data(), step, sizeof(int) * (nch + 1), cudaMemcpyDeviceToHost, st), "rows") ||
+      !ok(c, cudaMemcpyAsync(R.chunk_lo.data(), lohi, sizeof(int) * nch, cudaMemcpyDeviceToHost, st), "rows") ||
+      !ok(c, cudaMemcpyAsync(R.chunk_hi.data(), lohi + nch, sizeof(int) * nch, cudaMemcpyDeviceToHost, st), "rows") ||
+      !ok(c, cudaStreamSynchronize(st), "sync"))
+    return TG_ERR_CUDA;
+  const size_t slots = (size_t)R.chunk_step[nch] * 32;
+  int *blk = nullptr, *cidx = nullptr;
+  int2* slot = nullptr;
+  if (!dalloc(c, &blk, slots) || !dalloc(c, &cidx, slots) || !dalloc(c, &slot, slots)) return TG_ERR_OOM;
+  rows_chunk_kernel<true><<<grid, 256, 0, st>>>(R.rows, nch, node, c->d_rowptr, c->d_col, c->d_mask, rank, step, nullptr,
+                                                nullptr, blk, cidx);
+  c->launches += 3;
+  if (!ok(c, cudaGetLastError(), "rows kernels")) return TG_ERR_CUDA;
+  s = resident_slots(c, (long long)slots, blk, c->d_contrib_ptr, slot);
+  if (s) return s;
+  D.act_node = node;
+  D.blk = blk;
+  D.col = cidx;
+  D.chunk_step = step;
+  D.slot = slot;
+  D.contrib = c->d_contrib;
+  for (int* p : {flag, rank, tmp, cnt, lohi}) dfree(c, p);
+  return TG_OK;
+}
+}  // namespace
+
 // The mesh's buffers went back to the pool with it.
 void resident_reset(Context* c) {
   if (!c->res) return;
@@ -1108,11 +1472,30 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
       }
       M.plan_of.push_back(it->second);
     }
+  } else if (!batch) {
+    if (c->composed) return TG_OK;  // one solve over a composed batch: streamed
+    // a mesh above the chip's chunks is not looked at row by row
+    const int chunks = elem == 4 ? ResShape<float>::warps * ResShape<float>::slots
+                                 : ResShape<double>::warps * ResShape<double>::slots;
+    if ((long long)c->neq > 3LL * c->num_sms * chunks * kResChunkRows || c->neq == 0) return TG_OK;
+    ResRows R;
+    ResPlan P;
+    s = rows_of_mesh(c, R, P.dev);
+    if (s) return s;
+    if (!resident_plan(R, elem, c->num_sms, cap, cluster, true, P)) return TG_OK;
+    ResImage img;
+    const size_t at = img.split_at(P);
+    int* d = nullptr;
+    if (!dalloc(c, &d, img.data.size())) return TG_ERR_OOM;
+    if (!ok(c, cudaMemcpyAsync(d, img.data.data(), sizeof(int) * img.data.size(), cudaMemcpyHostToDevice, c->stream),
+            "resident split") ||
+        !ok(c, cudaStreamSynchronize(c->stream), "sync"))
+      return TG_ERR_CUDA;
+    resident_bind_split(P.dev, d, at, P);
+    M.plans.push_back(P);
+    M.plan_of.push_back(0);
   } else {
-    if (c->composed && !batch) return TG_OK;  // one solve over a composed batch: streamed
     if (ensure_host_mesh(c)) return TG_ERR_CUDA;
-    // a mesh far above the chip's shared memory is not looked at row by row
-    if (!batch && (double)c->nnzb * 9 * elem > 1.5 * (double)cap * c->num_sms) return TG_OK;
     std::vector<ResRows> rows(nseg);
     std::vector<uint8_t> mask(c->nnd, 0);
     for (int n = 0; n < c->nnd; ++n)
@@ -1121,10 +1504,10 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
     ResImage img;
     std::vector<size_t> at_rows(nseg), at_split(nseg);
     for (int i = 0; i < nseg; ++i) {
-      const int n0 = batch ? c->h_seg_node[i] : 0, n1 = batch ? c->h_seg_node[i + 1] : c->nnd;
+      const int n0 = c->h_seg_node[i], n1 = c->h_seg_node[i + 1];
       resident_rows(n0, n1, c->h_rowptr.data(), c->h_col.data(), mask.data(), rows[i]);
       ResPlan P;
-      if (!rows[i].act_node.empty() && !resident_plan(rows[i], elem, c->num_sms, cap, cluster, !batch, P)) return TG_OK;
+      if (!rows[i].act_node.empty() && !resident_plan(rows[i], elem, c->num_sms, cap, cluster, false, P)) return TG_OK;
       at_rows[i] = img.rows_at(rows[i]);
       at_split[i] = img.split_at(P);
       M.plans.push_back(P);
@@ -1179,19 +1562,18 @@ int grow(Context* c, T** p, long long* cap, long long n) {
   return TG_OK;
 }
 
+// Runs the solves of the listed RVEs (act; one for a whole mesh) for nvec
+// right-hand sides, nnd nodes apart in d_rhs and x, and reports each in out.
+// x is zero away from the solved rows.
 template <typename T>
-int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double rel_tol, int max_it, int precond,
-                     int* iters, double* rel_res) {
+int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>& act, const double4_32a* d_rhs, int nvec,
+                 typename Vec4<T>::type* x, double rel_tol, int max_it, int precond, std::vector<ResItem>& items,
+                 std::vector<ResOut>& out) {
   using V = typename Vec4<T>::type;
-  const bool batch = c->nseg > 0 && c->seg_pcg_mode;
-  const int precision = sizeof(T) == 4 ? TG_MIXED : TG_FP64;
   ResState& S = *c->res;
-  int s = pcg_vectors(c, precision);
-  if (s) return s;
+  int s = TG_OK;
   cudaStream_t st = c->stream;
-  const int nseg = batch ? c->nseg : 1;
-  std::vector<uint8_t> act(nseg, 1);
-  if (batch && (int)c->seg_active.size() == nseg) act = c->seg_active;
+  const int nseg = (int)act.size();
   // launch classes: grid solves together, cluster solves by (CTAs, warps,
   // shared memory), the longest first
   struct Class {
@@ -1216,10 +1598,10 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
     C.smem = std::max(C.smem, P.smem);
     C.seg.push_back(i);
   }
-  std::vector<ResItem> items;
-  auto add = [&](int i, long long ll) {
+  items.clear();
+  auto add = [&](int i, int vec, long long ll) {
     const int p = M.plan_of[i];
-    ResItem it{p, i, batch ? c->h_seg_node[i] : 0, 0, ll};
+    ResItem it{p, i, batch ? c->h_seg_node[i] : 0, 0, vec, 0, ll};
     // a template's contribution map counts its own elements; an uploaded
     // mesh's counts the mesh's
     if (batch && c->inst_segments) it.elem_off = c->h_seg_elem[i];
@@ -1230,11 +1612,12 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
     return ka != kb ? ka > kb : a < b;
   });
   long long ll = 0;
-  for (int i : grid_seg) {
-    const ResPlan& P = M.plans[M.plan_of[i]];
-    add(i, ll);
-    ll += 6LL * P.k * P.k + (long long)P.rows * RowWords<T>::n;
-  }
+  for (int i : grid_seg)
+    for (int v = 0; v < nvec; ++v) {
+      const ResPlan& P = M.plans[M.plan_of[i]];
+      add(i, v, ll);
+      ll += 4LL * std::min(P.k, kResCopies) * P.k + (long long)P.rows * RowWords<T>::n;
+    }
   // grid solves in waves: a wave's solves take disjoint CTAs, first fit
   std::vector<std::vector<int2>> lists;
   std::vector<int> sched;
@@ -1243,8 +1626,8 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
   {
     std::vector<int> used;
     std::vector<std::vector<std::pair<int, int>>> wave;  // (item, first CTA)
-    for (size_t q = 0; q < grid_seg.size(); ++q) {
-      const ResPlan& P = M.plans[M.plan_of[grid_seg[q]]];
+    for (size_t q = 0; q < items.size(); ++q) {
+      const ResPlan& P = M.plans[items[q].plan];
       size_t w = 0;
       while (w < used.size() && used[w] + P.k > c->num_sms) ++w;
       if (w == used.size()) {
@@ -1259,7 +1642,7 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
     if (!used.empty()) lists.resize(*std::max_element(used.begin(), used.end()));
     for (const auto& w : wave)
       for (const auto& e : w)
-        for (int r = 0; r < M.plans[M.plan_of[grid_seg[e.first]]].k; ++r)
+        for (int r = 0; r < M.plans[items[e.first].plan].k; ++r)
           lists[e.second + r].push_back(make_int2(e.first, r));
     int at = 0;
     for (const auto& l : lists) {
@@ -1276,7 +1659,8 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
   }
   const size_t n_grid = items.size();
   for (auto& e : cls)
-    for (int i : e.second.seg) add(i, 0);
+    for (int i : e.second.seg)
+      for (int v = 0; v < nvec; ++v) add(i, v, 0);
   const int n = (int)items.size();
   long long icap = S.items_cap, ocap = S.items_cap;
   s = grow(c, &S.d_items, &icap, n);
@@ -1289,7 +1673,7 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
     if (s) return s;
   }
   // rows outside every solve (prescribed nodes, RVEs not solved) stay zero
-  if (!ok(c, cudaMemsetAsync(c->d_x, 0, sizeof(V) * (size_t)c->nnd, st), "x") ||
+  if (!ok(c, cudaMemsetAsync(x, 0, sizeof(V) * (size_t)c->nnd * nvec, st), "x") ||
       !ok(c, cudaMemsetAsync(S.d_out, 0, sizeof(ResOut) * (size_t)std::max(n, 1), st), "out"))
     return TG_ERR_CUDA;
   if (n == 0) {
@@ -1309,7 +1693,8 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
   A.Ke = sizeof(T) == 4 ? (const T*)c->d_Ke32 : (const T*)c->d_Ke64;
   A.mask = c->d_mask;
   A.rhs = d_rhs;
-  A.x = (V*)c->d_x;
+  A.x = x;
+  A.nnd = c->nnd;
   A.out = S.d_out;
   A.ll = S.d_ll;
   A.sc = c->d_pcg;
@@ -1359,9 +1744,10 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
       B.items = S.d_items + first;
       B.out = S.d_out + first;
       B.k = C.k;
-      first += C.seg.size();
+      const size_t solves = C.seg.size() * (size_t)nvec;
+      first += solves;
       cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)(C.seg.size() * C.k));
+      cfg.gridDim = dim3((unsigned)(solves * C.k));
       cfg.blockDim = dim3(32u * (unsigned)C.warps);
       cfg.dynamicSmemBytes = C.smem;
       cfg.stream = q % nst == 0 ? st : S.aux[q % nst - 1];
@@ -1381,15 +1767,34 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
       if (!ok(c, cudaEventRecord(S.join[a], S.aux[a]), "join") || !ok(c, cudaStreamWaitEvent(st, S.join[a], 0), "join"))
         return TG_ERR_CUDA;
   }
-  std::vector<ResOut> out(std::max(n, 1));
+  out.assign(std::max(n, 1), ResOut{});
   if (n && !ok(c, cudaMemcpyAsync(out.data(), S.d_out, sizeof(ResOut) * n, cudaMemcpyDeviceToHost, st), "out"))
     return TG_ERR_CUDA;
   if (!ok(c, cudaStreamSynchronize(st), "pcg sync")) return TG_ERR_CUDA;
-  for (int i = 0; i < n; ++i)
-    if (out[i].done == 0) {  // a wait ran out before this solve reported
-      out[i].done = 2;
-      out[i].fail = 5;
+  out.resize(n);
+  for (ResOut& o : out)
+    if (o.done == 0) {  // a wait ran out before this solve reported
+      o.done = 2;
+      o.fail = 5;
     }
+  return TG_OK;
+}
+
+template <typename T>
+int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double rel_tol, int max_it, int precond,
+                     int* iters, double* rel_res) {
+  using V = typename Vec4<T>::type;
+  const bool batch = c->nseg > 0 && c->seg_pcg_mode;
+  int s = pcg_vectors(c, sizeof(T) == 4 ? TG_MIXED : TG_FP64);
+  if (s) return s;
+  const int nseg = batch ? c->nseg : 1;
+  std::vector<uint8_t> act(nseg, 1);
+  if (batch && (int)c->seg_active.size() == nseg) act = c->seg_active;
+  std::vector<ResItem> items;
+  std::vector<ResOut> out;
+  s = run_resident<T>(c, M, batch, act, d_rhs, 1, (V*)c->d_x, rel_tol, max_it, precond, items, out);
+  if (s) return s;
+  const int n = (int)items.size();
   if (!batch) {
     PcgScalars h;
     std::memset(&h, 0, sizeof(h));
@@ -1440,6 +1845,60 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
 }
 
 }  // namespace
+
+// w = v + x, nine vectors (x: the solutions on the free dofs, zero elsewhere)
+namespace {
+template <typename V>
+__global__ void resident_add_kernel(long long n, const double4_32a* __restrict__ v, const V* __restrict__ x,
+                                    double4_32a* __restrict__ w) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double4_32a a = v[i];
+  const V b = x[i];
+  w[i] = make_double4_32a(a.x + (double)b.x, a.y + (double)b.y, a.z + (double)b.z, 0.0);
+}
+
+template <typename T>
+int macro_resident_t(Context* c, ResMode& M, int nvec, const double4_32a* d_b, const double4_32a* d_v,
+                     double4_32a* d_w, double rel_tol, int max_it, int precond, int* iters) {
+  using V = typename Vec4<T>::type;
+  V* x = nullptr;
+  const long long nv = (long long)c->nnd * nvec;
+  if (!ok(c, cudaMallocAsync((void**)&x, sizeof(V) * (size_t)nv, c->stream), "alloc")) return TG_ERR_OOM;
+  std::vector<ResItem> items;
+  std::vector<ResOut> out;
+  int s = run_resident<T>(c, M, true, std::vector<uint8_t>(c->nseg, 1), d_b, nvec, x, rel_tol, max_it, precond, items,
+                          out);
+  if (!s) {
+    resident_add_kernel<V><<<(unsigned)((nv + 255) / 256), 256, 0, c->stream>>>(nv, d_v, x, d_w);
+    c->launches++;
+    if (!ok(c, cudaGetLastError(), "resident_add_kernel")) s = TG_ERR_CUDA;
+  }
+  cudaFreeAsync(x, c->stream);
+  if (s) return s;
+  int worst = 0, limit = 0;
+  static const char* why[] = {"", "non-finite initial residual", "p.Ap <= 0 (indefinite operator)", "p.Ap not finite",
+                              "non-finite update", "exchange wait timed out"};
+  for (const ResOut& o : out) {
+    worst = std::max(worst, o.iters);
+    if (o.done == 2) {
+      c->err = std::string("multi-vector PCG breakdown: ") + why[o.fail >= 0 && o.fail <= 5 ? o.fail : 0];
+      return TG_ERR_NAN;
+    }
+    limit += o.done == 3 ? 1 : 0;
+  }
+  if (iters) *iters = worst;
+  return limit ? TG_ERR_NOT_CONVERGED : TG_OK;
+}
+}  // namespace
+
+int macro_solve_resident(Context* c, int precision, int nvec, const double4_32a* d_b, const double4_32a* d_v,
+                         double4_32a* d_w, double rel_tol, int max_it, int precond, int* iters) {
+  ResMode& M = c->res->mode[precision == TG_MIXED ? 1 : 0][1];
+  return precision == TG_MIXED
+             ? macro_resident_t<float>(c, M, nvec, d_b, d_v, d_w, rel_tol, max_it, precond, iters)
+             : macro_resident_t<double>(c, M, nvec, d_b, d_v, d_w, rel_tol, max_it, precond, iters);
+}
 
 // The default form solves resident where the mesh (every RVE of the batch)
 // fits; the explicit forms of tg_pcg_form and the symmetric format keep their

@@ -24,9 +24,10 @@ struct ResPlanDev {
   int rows, k, nchunks;
 };
 
-// One solve of a launch: a plan applied at an instance's offsets.
+// One solve of a launch: a plan applied at an instance's offsets to one of the
+// call's right-hand sides.
 struct ResItem {
-  int plan, seg, node_off, elem_off;
+  int plan, seg, node_off, elem_off, vec, pad;
   long long ll;  // grid form: first word of its exchange area
 };
 
@@ -38,6 +39,7 @@ struct ResOut {
 
 // Rows of a mesh or RVE in the kernel's order (host).
 struct ResRows {
+  int rows = 0;
   std::vector<int> act_node, blk, col, chunk_step, chunk_lo, chunk_hi;
 };
 

@@ -475,6 +475,9 @@ void cg_free(Context* c);  // the captured iterations
 int resident_active(Context* c, int precision, bool* on);
 int pcg_solve_resident(Context* c, const double4_32a* d_rhs, double rel_tol, int max_it, int precond, int* iters,
                        double* rel_res);
+// nvec right-hand sides of every RVE of a batch: w = v + K^-1 b per RVE
+int macro_solve_resident(Context* c, int precision, int nvec, const double4_32a* d_b, const double4_32a* d_v,
+                         double4_32a* d_w, double rel_tol, int max_it, int precond, int* iters);
 void resident_reset(Context* c);
 void resident_drop_batch(Context* c);
 void resident_destroy(Context* c);
@@ -482,8 +485,9 @@ inline bool ke_current(const Context* c) {
   return (c->tangent_precision == TG_MIXED && c->ke_serial32 == c->tangent_serial) ||
          (c->tangent_precision == TG_FP64 && c->ke_serial64 == c->tangent_serial);
 }
-// rhs = R - K v from the element blocks, v zero away from prescribed dofs
-int launch_lift_elements(Context* c, const double4_32a* d_v, double4_32a* d_rhs);
+// rhs = R - K v from the element blocks, v zero away from prescribed dofs;
+// with zero_base, rhs = -K v for nvec vectors, nnd apart
+int launch_lift_elements(Context* c, const double4_32a* d_v, double4_32a* d_rhs, bool zero_base = false, int nvec = 1);
 // symmetric push storage: structure (once per mesh) and values of the last
 // assembly in the given precision (pushfmt.cu)
 int push_prepare(Context* c, int precision);
@@ -509,6 +513,7 @@ inline bool push_solve(const Context* c) {
   return c->pcg_form == 1 && !sym_active(c) && push_active(c);
 }
 void push_free(Context* c);
+int scan_counts(Context* c, int n, const int* d_in, int* d_out, int* d_tmp);  // d_tmp: n / 4096 + 3 ints
 int time_cg_kernel(Context* c, int which, int reps, double* ms);  // 0 product, 1 vector kernel
 // PCG with every work vector, partial sum and scalar in caller scratch
 constexpr size_t kScratchScalarBytes = 256;
