@@ -78,12 +78,17 @@ template <typename T>
 struct ResShape;
 template <>
 struct ResShape<float> {
-  static constexpr int warps = 16, slots = 4, reg = 7, off = 3, state = 6;
+  static constexpr int warps = 16, slots = 4, reg = 5, tm = 7, off = 3, state = 6;
 };
 template <>
 struct ResShape<double> {
-  static constexpr int warps = 16, slots = 1, reg = 0, off = 0, state = 0;
+  static constexpr int warps = 16, slots = 1, reg = 0, tm = 0, off = 0, state = 0;
 };
+// steps of chunk i of a part of nw warps that stay out of shared memory
+template <typename T>
+__host__ __device__ constexpr int res_off_steps(int i, int nw) {
+  return i < nw ? ResShape<T>::reg : i < ResShape<T>::off * nw ? ResShape<T>::tm : 0;
+}
 constexpr int kTmemColumns = 512;
 
 using u64 = unsigned long long;
@@ -561,37 +566,45 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
   const int row0 = ch0 * kResChunkRows, row1 = min(P.rows, (ch0 + nch) * kResChunkRows);
   // shared memory: the window [columns][4]; FP32: every chunk's p, s, x and
   // preconditioner [chunks][.][32]; the values that are in neither registers
-  // nor tensor memory [steps][9][32]; the columns of every step [steps][32]
+  // nor tensor memory [steps][9][32]; the columns, eight steps of a lane in
+  // one 16-byte word [groups][32][8] (padded with the chunk's first row)
   V* uw = reinterpret_cast<V*>(smem);
   const int steps0 = P.chunk_step[ch0];
-  int vstep[NS], cstep[NS], nst[NS];  // first value step, first index step, steps of this warp's chunks
-  int vsteps = 0;                     // value steps in shared memory
+  // this warp's chunks: first value step and column group in shared memory,
+  // steps, packed (the loop below is short of registers)
+  unsigned lay[NS];
+  auto vstep_of = [&](int q) { return (int)(lay[q] >> 20); };
+  auto cgrp_of = [&](int q) { return (int)((lay[q] >> 8) & 0xfffu); };
+  auto nst_of = [&](int q) { return (int)(lay[q] & 0xffu); };
+  int vsteps = 0;  // value steps in shared memory
   {
 #pragma unroll
-    for (int q = 0; q < NS; ++q) vstep[q] = cstep[q] = nst[q] = 0;
+    for (int q = 0; q < NS; ++q) lay[q] = 0u;
+    int groups = 0;
     for (int i0 = 0; i0 < nch; i0 += 32) {
       const int i = i0 + lane;
       const int b = i < nch ? P.chunk_step[ch0 + i] : 0, n = i < nch ? P.chunk_step[ch0 + i + 1] - b : 0;
-      const int v = i < OFF * nw ? max(0, n - RB) : n;
-      int inc = v;
+      const int v = max(0, n - res_off_steps<T>(i, nw)), gr = (n + 7) >> 3;
+      int inc = v, ging = gr;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
+        const int y = __shfl_up_sync(0xffffffffu, inc, o), z = __shfl_up_sync(0xffffffffu, ging, o);
+        if (lane >= o) {
+          inc += y;
+          ging += z;
+        }
       }
 #pragma unroll
       for (int q = 0; q < NS; ++q) {
         const int mine = warp + q * nw;  // this warp's chunk of slot q
         const int from = mine & 31;
-        const int ve = __shfl_sync(0xffffffffu, vsteps + inc - v, from), ce = __shfl_sync(0xffffffffu, b, from),
-                  ne = __shfl_sync(0xffffffffu, n, from);
-        if (mine < nch && mine >= i0 && mine < i0 + 32) {
-          vstep[q] = ve;
-          cstep[q] = ce - steps0;
-          nst[q] = ne;
-        }
+        const int ve = __shfl_sync(0xffffffffu, vsteps + inc - v, from), ne = __shfl_sync(0xffffffffu, n, from),
+                  ge = __shfl_sync(0xffffffffu, groups + ging - gr, from);
+        if (mine < nch && mine >= i0 && mine < i0 + 32)
+          lay[q] = ((unsigned)ve << 20) | ((unsigned)ge << 8) | (unsigned)ne;
       }
       vsteps += __shfl_sync(0xffffffffu, inc, 31);
+      groups += __shfl_sync(0xffffffffu, ging, 31);
     }
   }
   T* state = reinterpret_cast<T*>(uw + win.y);  // p, s, x
@@ -642,12 +655,13 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
         if (o != rank && row >= sh.peer[o].x && row < sh.peer[o].x + sh.peer[o].y) peers[q] |= 1u << o;
     T D[9];
     bool have = false;
+    const int step0 = i < nch ? P.chunk_step[ch0 + i] : 0, nst = nst_of(q), cgrp = cgrp_of(q);
     auto block = [&](int t, T acc[9]) {
-      const int at = (steps0 + cstep[q] + t) * 32 + lane;
+      const int at = (step0 + t) * 32 + lane;
       const int cl = P.col[at];
       const int2 sl = P.slot[at];
       slot_value<T>(sl, m, P.contrib, A.Ke, I.elem_off, acc);
-      cols[(size_t)(cstep[q] + t) * 32 + lane] = (uint16_t)(cl - win.x);
+      cols[((size_t)(cgrp + (t >> 3)) * 32 + lane) * 8 + (t & 7)] = (uint16_t)(cl - win.x);
       if (cl == row && sl.y > 0) {
         have = true;
 #pragma unroll
@@ -659,7 +673,7 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
     if (q == 0 && RB > 0) {
 #pragma unroll
       for (int t = 0; t < RB; ++t) {
-        if (t < nst[0]) {
+        if (t < nst) {
           block(t, rv[t]);
         } else {
 #pragma unroll
@@ -667,19 +681,29 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
         }
       }
     }
+    // the columns' padding: the chunk's first row
+    for (int t = nst; t < (nst + 7) / 8 * 8; ++t)
+      cols[((size_t)(cgrp + (t >> 3)) * 32 + lane) * 8 + (t & 7)] =
+          (uint16_t)((ch0 + i) * kResChunkRows - win.x);
     if constexpr (F32) {
-      if (q > 0 && q < OFF)
-        for (int t = 0; t < min(RB, nst[q]); ++t) {
+      if (q > 0 && q < OFF && nst > 0)
+        for (int t = 0; t < Shape::tm; ++t) {
           T acc[9];
-          block(t, acc);
+          if (t < nst) {
+            block(t, acc);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 9; ++e) acc[e] = T(0);
+          }
           __syncwarp();
           tmem_st9(tm + (unsigned)(q - 1) * 64u + 9u * (unsigned)t, acc);
         }
     }
-    for (int t = q < OFF ? RB : 0; t < nst[q]; ++t) {
+    const int off = q == 0 ? RB : q < OFF ? Shape::tm : 0;
+    for (int t = off; t < nst; ++t) {
       T acc[9];
       block(t, acc);
-      T* vp = vals + (size_t)(vstep[q] + t - (q < OFF ? RB : 0)) * 9 * 32 + lane;
+      T* vp = vals + (size_t)(vstep_of(q) + t - off) * 9 * 32 + lane;
 #pragma unroll
       for (int e = 0; e < 9; ++e) vp[32 * e] = acc[e];
     }
@@ -827,57 +851,86 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
     } else {
       __syncthreads();
     }
-    // w = A u, one chunk after the other
+    // w = A u, one chunk after the other: a lane's column indices of eight
+    // steps are one load, so a batch's gathers are all in flight together
+    // (indices read step by step left 5 wavefronts a step waiting on two
+    // dependent loads)
     T w[NS], A0[NS], A1[NS], A2[NS];
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
       A0[q] = A1[q] = A2[q] = T(0);
       if (q * nw >= nch) break;
       T a0 = T(0), a1 = T(0), a2 = T(0);
-      const uint16_t* cp = cols + (size_t)cstep[q] * 32 + lane;
-      if (q == 0 && RB > 0) {
-#pragma unroll
-        for (int t = 0; t < RB; ++t)
-          if (t < nst[0]) {
-            const V uj = uw[cp[32 * t]];
-            a0 += rv[t][0] * uj.x + rv[t][1] * uj.y + rv[t][2] * uj.z;
-            a1 += rv[t][3] * uj.x + rv[t][4] * uj.y + rv[t][5] * uj.z;
-            a2 += rv[t][6] * uj.x + rv[t][7] * uj.y + rv[t][8] * uj.z;
-          }
-      }
+      auto fma9 = [&](T m0, T m1, T m2, T m3, T m4, T m5, T m6, T m7, T m8, const V& uj) {
+        a0 += m0 * uj.x + m1 * uj.y + m2 * uj.z;
+        a1 += m3 * uj.x + m4 * uj.y + m5 * uj.z;
+        a2 += m6 * uj.x + m7 * uj.y + m8 * uj.z;
+      };
+      auto index = [](const uint4& g, int t) {
+        const unsigned v = t < 2 ? g.x : t < 4 ? g.y : t < 6 ? g.z : g.w;
+        return (t & 1) ? v >> 16 : v & 0xffffu;
+      };
+      const int nst = nst_of(q);
+      const uint4* cg = reinterpret_cast<const uint4*>(cols) + cgrp_of(q) * 32 + lane;
+      const T* vp = vals + vstep_of(q) * (9 * 32) + lane;
+      int t0 = 0;  // steps done
       if constexpr (F32) {
-        if (q > 0 && q < OFF) {
-          const unsigned col = tm + (unsigned)(q - 1) * 64u;
-          auto step = [&](int t, const unsigned* b) {
-            const V uj = uw[cp[32 * t]];
-            a0 += __uint_as_float(b[0]) * uj.x + __uint_as_float(b[1]) * uj.y + __uint_as_float(b[2]) * uj.z;
-            a1 += __uint_as_float(b[3]) * uj.x + __uint_as_float(b[4]) * uj.y + __uint_as_float(b[5]) * uj.z;
-            a2 += __uint_as_float(b[6]) * uj.x + __uint_as_float(b[7]) * uj.y + __uint_as_float(b[8]) * uj.z;
-          };
+        if (q < OFF) {
+          t0 = q == 0 ? RB : Shape::tm;
+          if (nst > 0) {
+            const uint4 g = *cg;
+            if (q == 0) {
+              auto batch = [&](auto from, auto to) {
+                constexpr int lo = decltype(from)::value, hi = decltype(to)::value;
+                V uj[4];
 #pragma unroll
-          for (int t = 0; t < RB; t += 2)
-            if (t < nst[q]) {
-              unsigned b[18];
-              __syncwarp();
-              if (t + 1 < RB)
-                tmem_ld18(col + 9u * (unsigned)t, b);
-              else
-                tmem_ld9(col + 9u * (unsigned)t, b);
-              tmem_wait_ld();
-              step(t, b);
-              if (t + 1 < RB && t + 1 < nst[q]) step(t + 1, b + 9);
+                for (int t = lo; t < hi; ++t) uj[t - lo] = uw[index(g, t)];
+#pragma unroll
+                for (int t = lo; t < hi; ++t)
+                  fma9(rv[t][0], rv[t][1], rv[t][2], rv[t][3], rv[t][4], rv[t][5], rv[t][6], rv[t][7], rv[t][8],
+                       uj[t - lo]);
+              };
+              batch(std::integral_constant<int, 0>{}, std::integral_constant<int, (RB < 4 ? RB : 4)>{});
+              if (RB > 4 && nst > 4) batch(std::integral_constant<int, 4>{}, std::integral_constant<int, RB>{});
+            } else {
+              const unsigned col = tm + (unsigned)(q - 1) * 64u;
+              auto pair = [&](auto at) {
+                constexpr int t = decltype(at)::value;
+                constexpr bool two = t + 1 < Shape::tm;
+                unsigned b[18];
+                __syncwarp();
+                if (two)
+                  tmem_ld18(col + 9u * (unsigned)t, b);
+                else
+                  tmem_ld9(col + 9u * (unsigned)t, b);
+                const V v0 = uw[index(g, t)];
+                V v1 = v0;
+                if (two) v1 = uw[index(g, t + 1)];
+                tmem_wait_ld();
+                auto f = [&](int e) { return __uint_as_float(b[e]); };
+                fma9(f(0), f(1), f(2), f(3), f(4), f(5), f(6), f(7), f(8), v0);
+                if (two) fma9(f(9), f(10), f(11), f(12), f(13), f(14), f(15), f(16), f(17), v1);
+              };
+              pair(std::integral_constant<int, 0>{});
+              pair(std::integral_constant<int, 2>{});
+              if (nst > 4) {
+                pair(std::integral_constant<int, 4>{});
+                pair(std::integral_constant<int, 6>{});
+              }
             }
+          }
         }
       }
-      const int t0 = q < OFF ? RB : 0;
-      cp += 32 * t0;
-      const T* vp = vals + (size_t)vstep[q] * 9 * 32 + lane;
-#pragma unroll 4
-      for (int t = t0; t < nst[q]; ++t, vp += 9 * 32, cp += 32) {
-        const V uj = uw[*cp];
-        a0 += vp[0] * uj.x + vp[32] * uj.y + vp[64] * uj.z;
-        a1 += vp[96] * uj.x + vp[128] * uj.y + vp[160] * uj.z;
-        a2 += vp[192] * uj.x + vp[224] * uj.y + vp[256] * uj.z;
+      for (; t0 < nst; t0 = (t0 | 7) + 1) {
+        const uint4 g = cg[(t0 >> 3) * 32];
+        const int e = min(nst, (t0 | 7) + 1);
+#pragma unroll
+        for (int t = 0; t < 8; ++t)
+          if ((t0 & ~7) + t >= t0 && (t0 & ~7) + t < e) {
+            const V uj = uw[index(g, t)];
+            fma9(vp[0], vp[32], vp[64], vp[96], vp[128], vp[160], vp[192], vp[224], vp[256], uj);
+            vp += 9 * 32;
+          }
       }
       A0[q] = a0;
       A1[q] = a1;
@@ -888,7 +941,7 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
 #pragma unroll
     for (int q = 0; q < NS; ++q) {
       w[q] = T(0);
-      if (q * nw >= nch) break;
+      if (q * nw >= nch) continue;
       const bool up = (c & 2) != 0;
       const T g0 = __shfl_xor_sync(0xffffffffu, up ? A0[q] : A2[q], 2);
       const T g1 = __shfl_xor_sync(0xffffffffu, A1[q], 2);
@@ -916,26 +969,52 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
     __syncthreads();
     if (sh.code) break;
     const T al = sh.coef[0], be = sh.coef[1];
+    if constexpr (F32) {
+      // two chunks at a time, loads first: the stores of one would order the
+      // next one's loads behind them
 #pragma unroll
-    for (int q = 0; q < NS; ++q) {
-      if (q * nw >= nch) break;
-      if (F32) {
-        T* sq = state + (size_t)(warp + q * nw) * 3 * 32 + lane;
-        if (warp + q * nw < nch) {
-          const T pn = u[q] + be * sq[0], sn = w[q] + be * sq[32];
-          sq[64] += al * pn;
-          sq[0] = pn;
-          sq[32] = sn;
-          r[q] -= al * sn;
+      for (int q2 = 0; q2 < NS; q2 += 2) {
+        if (q2 * nw >= nch) break;
+        T po[2], so[2], xo[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = warp + (q2 + h) * nw;
+          const T* sq = state + i * (3 * 32) + lane;
+          const bool on = i < nch;
+          po[h] = on ? sq[0] : T(0);
+          so[h] = on ? sq[32] : T(0);
+          xo[h] = on ? sq[64] : T(0);
         }
-      } else {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int q = q2 + h;
+          po[h] = u[q] + be * po[h];
+          so[h] = w[q] + be * so[h];
+          xo[h] += al * po[h];
+          r[q] -= al * so[h];
+          u[q] = precond(q, r[q]);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int i = warp + (q2 + h) * nw;
+          T* sq = state + i * (3 * 32) + lane;
+          if (i < nch) {
+            sq[0] = po[h];
+            sq[32] = so[h];
+            sq[64] = xo[h];
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < NS; ++q) {
+        if (q * nw >= nch) break;
         pr[q] = u[q] + be * pr[q];
         sr[q] = w[q] + be * sr[q];
         xr[q] += al * pr[q];
         r[q] -= al * sr[q];
+        u[q] = precond(q, r[q]);
       }
-      __syncwarp();
-      u[q] = precond(q, r[q]);
     }
   }
   const double unscale = power_of_two(-scale_exp);
@@ -1197,21 +1276,21 @@ void resident_rows(int n0, int n1, const int* rowptr, const int* col, const uint
 namespace {
 
 // Bytes of one part with nw warps: the window, FP32's vectors and
-// preconditioner, the values outside registers and tensor memory (the first
-// off * nw chunks keep `reg` steps there), the columns of every step.
-size_t part_bytes(const ResRows& R, int a, int b, int elem, int reg, int off, int state, int nw, int* lo, int* hi) {
+// preconditioner, the values outside registers and tensor memory (res_off_steps), the columns in groups of eight steps.
+size_t part_bytes(const ResRows& R, int a, int b, int elem, int nw, int* lo, int* hi) {
   int l = R.chunk_lo[a], h = R.chunk_hi[a];
-  size_t vsteps = 0;
+  const int state = elem == 4 ? ResShape<float>::state : ResShape<double>::state;
+  size_t vsteps = 0, groups = 0;
   for (int ch = a; ch < b; ++ch) {
     l = std::min(l, R.chunk_lo[ch]);
     h = std::max(h, R.chunk_hi[ch]);
     const int n = R.chunk_step[ch + 1] - R.chunk_step[ch];
-    vsteps += ch - a < off * nw ? std::max(0, n - reg) : n;
+    vsteps += std::max(0, n - (elem == 4 ? res_off_steps<float>(ch - a, nw) : res_off_steps<double>(ch - a, nw)));
+    groups += (n + 7) / 8;
   }
   *lo = l;
   *hi = h;
-  const size_t steps = (size_t)(R.chunk_step[b] - R.chunk_step[a]);
-  return (size_t)(h - l) * 4 * elem + (size_t)(b - a) * state * 32 * elem + vsteps * 9 * 32 * elem + steps * 64;
+  return (size_t)(h - l) * 4 * elem + (size_t)(b - a) * state * 32 * elem + vsteps * 9 * 32 * elem + groups * 512;
 }
 
 // The chunks cut into k consecutive parts of near-equal work; false if one
@@ -1221,9 +1300,6 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
   if (k > nch) return false;
   const int warps = elem == 4 ? ResShape<float>::warps : ResShape<double>::warps;
   const int slots = elem == 4 ? ResShape<float>::slots : ResShape<double>::slots;
-  const int reg = elem == 4 ? ResShape<float>::reg : ResShape<double>::reg;
-  const int off = elem == 4 ? ResShape<float>::off : ResShape<double>::off;
-  const int state = elem == 4 ? ResShape<float>::state : ResShape<double>::state;
   // a chunk's work is its steps and its vector updates (about two steps')
   auto work = [&](int ch) { return (long long)R.chunk_step[ch] + 2LL * ch; };
   const long long total = work(nch);
@@ -1245,7 +1321,8 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
   }
   P.part_win.assign(k, make_int4(0, 0, 0, 0));
   P.smem = 0;
-  int most = 0;
+  int most = 0, longest = 0;
+  for (int ch = 0; ch < nch; ++ch) longest = std::max(longest, R.chunk_step[ch + 1] - R.chunk_step[ch]);
   for (int q = 0; q < k; ++q) most = std::max(most, P.part_chunk[q + 1] - P.part_chunk[q]);
   if (most > warps * slots) return false;
   // one chunk per warp while there are warps for it
@@ -1253,8 +1330,9 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
   for (int q = 0; q < k; ++q) {
     const int a = P.part_chunk[q], b = P.part_chunk[q + 1];
     int lo, hi;
-    const size_t bytes = part_bytes(R, a, b, elem, reg, off, state, P.warps, &lo, &hi);
-    if (bytes > cap || hi - lo > 65535) return false;
+    const size_t bytes = part_bytes(R, a, b, elem, P.warps, &lo, &hi);
+    // (the kernel packs a chunk's steps, groups and value steps in 8, 12 and 12 bits)
+    if (bytes > cap || hi - lo > 65535 || longest > 255) return false;
     P.smem = std::max(P.smem, bytes);
     P.part_win[q] = make_int4(lo, hi - lo, q, q);
   }
