@@ -16,8 +16,8 @@
 //            partial sums travel through L2 as 16-byte words that carry their
 //            sequence number, so a reader polls the data itself and no
 //            barrier, flag or fence stands between producer and consumer.
-//            Larger RVEs of a batch share one launch: every CTA walks its
-//            list of (solve, part) pairs in one global order.
+//            A batch's larger RVEs are one launch per size, its groups of k
+//            CTAs dealing the solves.
 //
 // The recurrences are the single-reduction form of CG (Chronopoulos & Gear,
 // J. Comput. Appl. Math. 25 (1989) 153-168) as in pcg_cg.cu and segpcg.cu:
@@ -243,9 +243,8 @@ template <typename T>
 struct ResArgs {
   const ResPlanDev* plans;
   const ResItem* items;
-  const int* sched_ptr;  // grid form: CTA's first (item, part) pair
-  const int2* sched;
-  int k;                 // cluster form: CTAs per solve
+  int k;                 // CTAs per solve
+  int count;             // grid form: solves, dealt to the launch's groups of k CTAs
   const T* Ke;
   const uint8_t* mask;
   const double4_32a* rhs;
@@ -1083,9 +1082,9 @@ __global__ void __launch_bounds__(ResShape<T>::warps * 32, 1) resident_grid_kern
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ ResShared<T> sh;
   const bool tmem = tmem_begin(sh);
-  for (int e = A.sched_ptr[blockIdx.x]; e < A.sched_ptr[blockIdx.x + 1]; ++e) {
-    const int2 w = A.sched[e];
-    resident_solve<T, true, BLK>(A, A.items[w.x], w.x, w.y, smem, sh);
+  const int groups = gridDim.x / A.k, rank = blockIdx.x % A.k;
+  for (int item = blockIdx.x / A.k; item < A.count; item += groups) {
+    resident_solve<T, true, BLK>(A, A.items[item], item, rank, smem, sh);
     const bool stop = sh.abort_flag != 0;
     __syncthreads();
     if (stop) break;  // a wait ran out: nothing more is awaited
@@ -1496,8 +1495,6 @@ void resident_reset(Context* c) {
   S.items_cap = 0;
   S.d_ll = nullptr;
   S.ll_cap = 0;
-  S.d_sched = nullptr;
-  S.sched_cap = 0;
 }
 
 void resident_destroy(Context* c) {
@@ -1652,102 +1649,46 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
   int s = TG_OK;
   cudaStream_t st = c->stream;
   const int nseg = (int)act.size();
-  // launch classes: grid solves together, cluster solves by (CTAs, warps,
-  // shared memory), the longest first
+  // launch classes by form, CTAs, warps and shared memory, the largest first
   struct Class {
+    bool grid;
     int k, warps;
     size_t smem;
     std::vector<int> seg;
   };
   std::map<std::vector<long long>, Class> cls;
-  std::vector<int> grid_seg;
   for (int i = 0; i < nseg; ++i) {
     const ResPlan& P = M.plans[M.plan_of[i]];
     if (!act[i] || P.rows == 0) continue;
-    if (P.grid) {
-      grid_seg.push_back(i);
-      continue;
-    }
-    const int w = P.warps;
     const long long b = (long long)((P.smem + 16383) / 16384);
-    Class& C = cls[{-(long long)P.k, -w, -b}];
+    Class& C = cls[{P.grid ? 0 : 1, -(long long)P.k, -P.warps, -b}];
+    C.grid = P.grid;
     C.k = P.k;
-    C.warps = w;
+    C.warps = P.warps;
     C.smem = std::max(C.smem, P.smem);
     C.seg.push_back(i);
   }
   items.clear();
-  auto add = [&](int i, int vec, long long ll) {
-    const int p = M.plan_of[i];
-    ResItem it{p, i, batch ? c->h_seg_node[i] : 0, 0, vec, 0, ll};
-    // a template's contribution map counts its own elements; an uploaded
-    // mesh's counts the mesh's
-    if (batch && c->inst_segments) it.elem_off = c->h_seg_elem[i];
-    items.push_back(it);
-  };
-  std::sort(grid_seg.begin(), grid_seg.end(), [&](int a, int b) {
-    const int ka = M.plans[M.plan_of[a]].k, kb = M.plans[M.plan_of[b]].k;
-    return ka != kb ? ka > kb : a < b;
-  });
-  long long ll = 0;
-  for (int i : grid_seg)
-    for (int v = 0; v < nvec; ++v) {
-      const ResPlan& P = M.plans[M.plan_of[i]];
-      add(i, v, ll);
-      ll += 4LL * std::min(P.k, kResCopies) * P.k + (long long)P.rows * RowWords<T>::n;
-    }
-  // grid solves in waves: a wave's solves take disjoint CTAs, first fit
-  std::vector<std::vector<int2>> lists;
-  std::vector<int> sched;
-  int grid_warps = 0;
-  size_t grid_smem = 0;
-  {
-    std::vector<int> used;
-    std::vector<std::vector<std::pair<int, int>>> wave;  // (item, first CTA)
-    for (size_t q = 0; q < items.size(); ++q) {
-      const ResPlan& P = M.plans[items[q].plan];
-      size_t w = 0;
-      while (w < used.size() && used[w] + P.k > c->num_sms) ++w;
-      if (w == used.size()) {
-        used.push_back(0);
-        wave.emplace_back();
-      }
-      wave[w].push_back({(int)q, used[w]});
-      used[w] += P.k;
-      grid_warps = std::max(grid_warps, P.warps);
-      grid_smem = std::max(grid_smem, P.smem);
-    }
-    if (!used.empty()) lists.resize(*std::max_element(used.begin(), used.end()));
-    for (const auto& w : wave)
-      for (const auto& e : w)
-        for (int r = 0; r < M.plans[items[e.first].plan].k; ++r)
-          lists[e.second + r].push_back(make_int2(e.first, r));
-    int at = 0;
-    for (const auto& l : lists) {
-      sched.push_back(at);
-      at += (int)l.size();
-    }
-    sched.push_back(at);
-    if (sched.size() & 1) sched.push_back(0);  // the pairs are 8-byte aligned
-    for (const auto& l : lists)
-      for (const int2& e : l) {
-        sched.push_back(e.x);
-        sched.push_back(e.y);
-      }
-  }
-  const size_t n_grid = items.size();
+  long long ll = 0;  // exchange words of the grid solves
   for (auto& e : cls)
     for (int i : e.second.seg)
-      for (int v = 0; v < nvec; ++v) add(i, v, 0);
+      for (int v = 0; v < nvec; ++v) {
+        const ResPlan& P = M.plans[M.plan_of[i]];
+        ResItem it{M.plan_of[i], i, batch ? c->h_seg_node[i] : 0, 0, v, 0, ll};
+        // a template's contribution map counts its own elements; an uploaded
+        // mesh's counts the mesh's
+        if (batch && c->inst_segments) it.elem_off = c->h_seg_elem[i];
+        if (P.grid) ll += 4LL * std::min(P.k, kResCopies) * P.k + (long long)P.rows * RowWords<T>::n;
+        items.push_back(it);
+      }
   const int n = (int)items.size();
   long long icap = S.items_cap, ocap = S.items_cap;
   s = grow(c, &S.d_items, &icap, n);
   if (!s) s = grow(c, &S.d_out, &ocap, n);
   if (s) return s;
   S.items_cap = (int)icap;
-  if (n_grid) {
+  if (ll) {
     s = grow(c, &S.d_ll, &S.ll_cap, ll);
-    if (!s) s = grow(c, &S.d_sched, &S.sched_cap, (long long)sched.size());
     if (s) return s;
   }
   // rows outside every solve (prescribed nodes, RVEs not solved) stay zero
@@ -1765,9 +1706,7 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
   ResArgs<T> A;
   A.plans = M.d_plans;
   A.items = S.d_items;
-  A.sched_ptr = nullptr;
-  A.sched = nullptr;
-  A.k = 0;
+  A.k = A.count = 0;
   A.Ke = sizeof(T) == 4 ? (const T*)c->d_Ke32 : (const T*)c->d_Ke64;
   A.mask = c->d_mask;
   A.rhs = d_rhs;
@@ -1781,70 +1720,56 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
   const bool blk = precond == TG_PRECOND_BLOCK_JACOBI;
   A.max_it = max_it;
   A.tol = rel_tol;
-  if (n_grid) {
-    if (!ok(c, cudaMemcpyAsync(S.d_sched, sched.data(), sizeof(int) * sched.size(), cudaMemcpyHostToDevice, st),
-            "schedule") ||
-        !ok(c, cudaMemsetAsync(S.d_ll, 0, sizeof(uint4) * (size_t)ll, st), "exchange"))
-      return TG_ERR_CUDA;
-    ResArgs<T> G = A;
-    G.sched_ptr = S.d_sched;
-    G.sched = reinterpret_cast<const int2*>(S.d_sched + (lists.size() + 2) / 2 * 2);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)lists.size());
-    cfg.blockDim = dim3(32u * (unsigned)grid_warps);
-    cfg.dynamicSmemBytes = grid_smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    c->launches++;
-    if (!ok(c, cudaLaunchKernelEx(&cfg, blk ? resident_grid_kernel<T, true> : resident_grid_kernel<T, false>, G),
-            "resident_grid_kernel"))
-      return TG_ERR_CUDA;
+  if (ll && !ok(c, cudaMemsetAsync(S.d_ll, 0, sizeof(uint4) * (size_t)ll, st), "exchange")) return TG_ERR_CUDA;
+  // the classes run beside each other: each is small beside the chip's tail
+  // otherwise
+  const int naux = (int)std::min<size_t>(std::max<size_t>(cls.size(), 1) - 1, kResAux);
+  if (naux > 0) {
+    s = aux_streams(c);
+    if (s) return s;
+    if (!ok(c, cudaEventRecord(S.fork, st), "fork")) return TG_ERR_CUDA;
+    for (int q = 0; q < naux; ++q)
+      if (!ok(c, cudaStreamWaitEvent(S.aux[q], S.fork, 0), "fork")) return TG_ERR_CUDA;
   }
-  if (!cls.empty()) {
-    // classes side by side: each is small beside the chip's tail otherwise
-    const int nst = (int)std::min<size_t>(cls.size(), 4);
-    if (nst > 1) {
-      s = aux_streams(c);
-      if (s) return s;
-      if (!ok(c, cudaEventRecord(S.fork, st), "fork")) return TG_ERR_CUDA;
-      for (int q = 0; q + 1 < nst; ++q)
-        if (!ok(c, cudaStreamWaitEvent(S.aux[q], S.fork, 0), "fork")) return TG_ERR_CUDA;
-    }
-    size_t first = n_grid;
-    int q = 0;
-    for (const auto& e : cls) {
-      const Class& C = e.second;
-      ResArgs<T> B = A;
-      B.items = S.d_items + first;
-      B.out = S.d_out + first;
-      B.k = C.k;
-      const size_t solves = C.seg.size() * (size_t)nvec;
-      first += solves;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)(solves * C.k));
-      cfg.blockDim = dim3(32u * (unsigned)C.warps);
-      cfg.dynamicSmemBytes = C.smem;
-      cfg.stream = q % nst == 0 ? st : S.aux[q % nst - 1];
-      cudaLaunchAttribute at[1];
+  size_t first = 0;
+  int q = 0;
+  for (const auto& e : cls) {
+    const Class& C = e.second;
+    const size_t solves = C.seg.size() * (size_t)nvec;
+    ResArgs<T> B = A;
+    B.items = S.d_items + first;
+    B.out = S.d_out + first;
+    B.k = C.k;
+    B.count = (int)solves;
+    first += solves;
+    cudaLaunchConfig_t cfg = {};
+    // a cooperative launch holds as many groups of k CTAs as the chip at once
+    const size_t groups = C.grid ? std::min<size_t>(solves, std::max(1, c->num_sms / C.k)) : solves;
+    cfg.gridDim = dim3((unsigned)(groups * C.k));
+    cfg.blockDim = dim3(32u * (unsigned)C.warps);
+    cfg.dynamicSmemBytes = C.smem;
+    cfg.stream = q % (naux + 1) ? S.aux[q % (naux + 1) - 1] : st;
+    cudaLaunchAttribute at[1];
+    if (C.grid) {
+      at[0].id = cudaLaunchAttributeCooperative;
+      at[0].val.cooperative = 1;
+    } else {
       at[0].id = cudaLaunchAttributeClusterDimension;
       at[0].val.clusterDim.x = (unsigned)C.k;
       at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      c->launches++;
-      if (!ok(c, cudaLaunchKernelEx(&cfg, blk ? resident_cluster_kernel<T, true> : resident_cluster_kernel<T, false>, B),
-              "resident_cluster_kernel"))
-        return TG_ERR_CUDA;
-      ++q;
     }
-    for (int a = 0; a + 1 < nst; ++a)
-      if (!ok(c, cudaEventRecord(S.join[a], S.aux[a]), "join") || !ok(c, cudaStreamWaitEvent(st, S.join[a], 0), "join"))
-        return TG_ERR_CUDA;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    c->launches++;
+    auto* fn = C.grid ? (blk ? resident_grid_kernel<T, true> : resident_grid_kernel<T, false>)
+                      : (blk ? resident_cluster_kernel<T, true> : resident_cluster_kernel<T, false>);
+    if (!ok(c, cudaLaunchKernelEx(&cfg, fn, B), C.grid ? "resident_grid_kernel" : "resident_cluster_kernel"))
+      return TG_ERR_CUDA;
+    ++q;
   }
+  for (int a = 0; a < naux; ++a)
+    if (!ok(c, cudaEventRecord(S.join[a], S.aux[a]), "join") || !ok(c, cudaStreamWaitEvent(st, S.join[a], 0), "join"))
+      return TG_ERR_CUDA;
   out.assign(std::max(n, 1), ResOut{});
   if (n && !ok(c, cudaMemcpyAsync(out.data(), S.d_out, sizeof(ResOut) * n, cudaMemcpyDeviceToHost, st), "out"))
     return TG_ERR_CUDA;

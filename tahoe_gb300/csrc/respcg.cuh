@@ -9,6 +9,8 @@ namespace tg {
 
 constexpr int kResChunkRows = 8;  // rows of one warp, four lanes each
 
+constexpr int kResAux = 7;  // streams of a batch's cluster classes beside the context's own
+
 // One group's structure on the device: the active rows (nodes with a free
 // dof) of a mesh or of one RVE, their blocks in sliced-ELL order and their
 // split over CTAs.
@@ -71,10 +73,8 @@ struct ResState {
   int items_cap = 0;
   uint4* d_ll = nullptr;
   long long ll_cap = 0;
-  int* d_sched = nullptr;  // grid form: list starts, then (solve, part) pairs
-  long long sched_cap = 0;
-  cudaStream_t aux[3] = {nullptr, nullptr, nullptr};
-  cudaEvent_t fork = nullptr, join[3] = {nullptr, nullptr, nullptr};
+  cudaStream_t aux[kResAux] = {};
+  cudaEvent_t fork = nullptr, join[kResAux] = {};
   bool limits_known[2] = {false, false};
   size_t smem[2] = {0, 0};
   int cluster[2] = {1, 1};

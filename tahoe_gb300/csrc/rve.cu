@@ -2,7 +2,7 @@
 //
 // A batch of independent RVEs is uploaded as one disconnected mesh; RVE r owns
 // nodes [node_off[r], node_off[r+1]) and elements [elem_off[r], elem_off[r+1]).
-// One CTA per RVE reduces over its range in a fixed order (no atomics):
+// Their ranges are reduced in shares of a fixed size, a fixed order (no atomics):
 //  * segment_norms_kernel: ||R_r||^2 of the residual restricted to the RVE;
 //  * segment_stress_kernel: sum over the RVE's element nodes of fint (x) X,
 //    which is the integral of the first Piola stress over the RVE (the
@@ -40,42 +40,82 @@ __device__ __forceinline__ void cta_sum(double (&v)[NV]) {
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) segment_norms_kernel(int nseg, const int* __restrict__ off,
-                                                            const double4_32a* __restrict__ R, double* __restrict__ out) {
-  for (int sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
-    double v[1] = {0.0};
-    for (int n = off[sg] + threadIdx.x; n < off[sg + 1]; n += blockDim.x) {
-      const double4_32a r = R[n];
-      v[0] += r.x * r.x + r.y * r.y + r.z * r.z;
-    }
-    cta_sum<1>(v);
-    if (threadIdx.x == 0) out[sg] = v[0];
+// The ranges of the segments cut into shares of kShare entries, one CTA per
+// share: segment sg's shares are numbered from off[sg] / kShare + sg on, so
+// they depend on nothing but the offsets (a segment's sum has the same shares
+// in every batch).  The last share of a block number past its segment's end is
+// empty.  FP64 sums run at 2 lanes per cycle and SM here: one CTA per segment
+// took 0.5 ms for the stress of an RVE of side 24.
+template <int kShare>
+__device__ __forceinline__ bool share_of(int b, int nseg, const int* __restrict__ off, int& sg, int& e0, int& e1) {
+  int lo = 0, hi = nseg;  // the last segment whose first share is at most b
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (off[mid] / kShare + mid <= b)
+      lo = mid;
+    else
+      hi = mid;
   }
+  sg = lo;
+  e0 = off[lo] + (b - (off[lo] / kShare + lo)) * kShare;
+  e1 = min(off[lo + 1], e0 + kShare);
+  return e0 < e1;
+}
+inline int share_blocks(int total, int nseg, int share) { return total / share + nseg; }
+
+// out[sg][v] = the sum of its shares' partials in order
+template <int NV, int kShare>
+__global__ void segment_combine_kernel(int nseg, const int* __restrict__ off, const double* __restrict__ part,
+                                       double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nseg * NV) return;
+  const int sg = i / NV, v = i % NV;
+  const int b0 = off[sg] / kShare + sg, n = (off[sg + 1] - off[sg] + kShare - 1) / kShare;
+  double a = 0.0;
+  for (int b = 0; b < n; ++b) a += part[(long long)(b0 + b) * NV + v];
+  out[i] = a;
+}
+
+constexpr int kNormShare = 2048;   // nodes
+constexpr int kStressShare = 256;  // elements
+
+__global__ void __launch_bounds__(256) segment_norms_kernel(int nseg, const int* __restrict__ off,
+                                                            const double4_32a* __restrict__ R,
+                                                            double* __restrict__ part) {
+  int sg, n0, n1;
+  if (!share_of<kNormShare>(blockIdx.x, nseg, off, sg, n0, n1)) return;
+  double v[1] = {0.0};
+  for (int n = n0 + threadIdx.x; n < n1; n += blockDim.x) {
+    const double4_32a r = R[n];
+    v[0] += r.x * r.x + r.y * r.y + r.z * r.z;
+  }
+  cta_sum<1>(v);
+  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
 }
 
 __global__ void __launch_bounds__(256) segment_stress_kernel(int nseg, const int* __restrict__ eoff,
                                                              const int* __restrict__ conn, const double* __restrict__ X,
                                                              int nnd, const double4_32a* __restrict__ fint,
-                                                             double* __restrict__ out) {
-  for (int sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
-    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const long long k0 = (long long)eoff[sg] * 8, k1 = (long long)eoff[sg + 1] * 8;
-    for (long long k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-      const int n = conn[k];
-      const double4_32a f = fint[k];
-      const double Xn[3] = {X[n], X[nnd + n], X[2 * nnd + n]};
+                                                             double* __restrict__ part) {
+  int sg, e0, e1;
+  if (!share_of<kStressShare>(blockIdx.x, nseg, eoff, sg, e0, e1)) return;
+  double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  const long long k1 = (long long)e1 * 8;
+  for (long long k = (long long)e0 * 8 + threadIdx.x; k < k1; k += blockDim.x) {
+    const int n = conn[k];
+    const double4_32a f = fint[k];
+    const double Xn[3] = {X[n], X[nnd + n], X[2 * nnd + n]};
 #pragma unroll
-      for (int J = 0; J < 3; ++J) {
-        v[0 * 3 + J] += f.x * Xn[J];
-        v[1 * 3 + J] += f.y * Xn[J];
-        v[2 * 3 + J] += f.z * Xn[J];
-      }
+    for (int J = 0; J < 3; ++J) {
+      v[0 * 3 + J] += f.x * Xn[J];
+      v[1 * 3 + J] += f.y * Xn[J];
+      v[2 * 3 + J] += f.z * Xn[J];
     }
-    cta_sum<9>(v);
-    if (threadIdx.x == 0)
-#pragma unroll
-      for (int k = 0; k < 9; ++k) out[(long long)sg * 9 + k] = v[k];
   }
+  cta_sum<9>(v);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < 9; ++k) part[(long long)blockIdx.x * 9 + k] = v[k];
 }
 
 // v = (e_k (x) e_L) X on prescribed dofs, zero elsewhere: the boundary
@@ -191,16 +231,28 @@ int launch_segment_macro(Context* c, const double4_32a* d_w, int kL, int ncols, 
 }
 
 int launch_segment_norms(Context* c, int nseg, const int* d_node_off, double* d_out) {
-  segment_norms_kernel<<<std::min(nseg, c->num_sms * 16), 256, 0, c->stream>>>(nseg, d_node_off, c->d_R, d_out);
-  c->launches++;
-  return ok(c, cudaGetLastError(), "segment_norms_kernel") ? TG_OK : TG_ERR_CUDA;
+  const int nb = share_blocks(c->nnd, nseg, kNormShare);
+  double* part = nullptr;
+  if (!ok(c, cudaMallocAsync((void**)&part, sizeof(double) * nb, c->stream), "alloc")) return TG_ERR_OOM;
+  segment_norms_kernel<<<nb, 256, 0, c->stream>>>(nseg, d_node_off, c->d_R, part);
+  segment_combine_kernel<1, kNormShare><<<(nseg + 127) / 128, 128, 0, c->stream>>>(nseg, d_node_off, part, d_out);
+  c->launches += 2;
+  const int s = ok(c, cudaGetLastError(), "segment_norms_kernel") ? TG_OK : TG_ERR_CUDA;
+  cudaFreeAsync(part, c->stream);
+  return s;
 }
 
 int launch_segment_stress(Context* c, int nseg, const int* d_elem_off, double* d_out) {
-  segment_stress_kernel<<<std::min(nseg, c->num_sms * 16), 256, 0, c->stream>>>(nseg, d_elem_off, c->d_conn, c->d_X,
-                                                                              c->nnd, c->d_fint, d_out);
-  c->launches++;
-  return ok(c, cudaGetLastError(), "segment_stress_kernel") ? TG_OK : TG_ERR_CUDA;
+  const int nb = share_blocks(c->nel, nseg, kStressShare);
+  double* part = nullptr;
+  if (!ok(c, cudaMallocAsync((void**)&part, sizeof(double) * 9 * nb, c->stream), "alloc")) return TG_ERR_OOM;
+  segment_stress_kernel<<<nb, 256, 0, c->stream>>>(nseg, d_elem_off, c->d_conn, c->d_X, c->nnd, c->d_fint, part);
+  segment_combine_kernel<9, kStressShare>
+      <<<(nseg * 9 + 127) / 128, 128, 0, c->stream>>>(nseg, d_elem_off, part, d_out);
+  c->launches += 2;
+  const int s = ok(c, cudaGetLastError(), "segment_stress_kernel") ? TG_OK : TG_ERR_CUDA;
+  cudaFreeAsync(part, c->stream);
+  return s;
 }
 
 }  // namespace tg
