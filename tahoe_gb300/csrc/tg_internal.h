@@ -441,6 +441,9 @@ template <typename G>
 int launch_geometry(Context* c, const double* X, int nnd, const int* conn, int nel, G* geo, long long stride,
                     long long off);
 int launch_tangent(Context* c, int precision);   // Ke per element
+// the same for moduli of the isotropic form (tangent_iso.cu)
+bool tangent_iso_applies(const Context* c, int precision);
+int launch_tangent_iso(Context* c);
 int launch_assemble(Context* c, int precision);
 int launch_blob_structure(Context* c, int precision);
 // segmented (per-RVE) reductions over node / element ranges
