@@ -59,7 +59,7 @@ struct ResPlan {
 // The plans of the current mesh for one precision, for a solve of the whole
 // mesh or of its RVEs.
 struct ResMode {
-  int state = 0;  // 0 not planned, 1 resident, -1 does not fit
+  int state = 0;  // 0 not planned, 1 resident, 2 hybrid, -1 neither
   std::vector<ResPlan> plans;
   std::vector<int> plan_of;  // plan of every RVE (one entry for a whole mesh)
   ResPlanDev* d_plans = nullptr;

@@ -71,6 +71,7 @@ struct ResidScalars {
   int pad;
 };
 
+struct HybState;      // plan and buffers of the hybrid PCG (hybridpcg.cu)
 struct ResState;      // plans and buffers of the resident PCG (respcg.cuh)
 struct MeshTemplate;  // a resident template mesh (compose.cu)
 // geometry planes (25 planes of 8 points per element) of every resident
@@ -242,6 +243,7 @@ struct Context {
   long long tangent_serial = 0; // assemblies so far (values of derived storages follow it)
   long long ke_serial32 = -1, ke_serial64 = -1;      // tangent serial of the element blocks on the device
   ResState* res = nullptr;
+  HybState* hyb = nullptr;
   long long full_serial32 = -1, full_serial64 = -1;  // tangent serial of the full storage's values
   int* d_contrib_ptr = nullptr; // nnzb+1
   int* d_contrib = nullptr;     // nel*64: e*64 + a*8 + b
@@ -481,6 +483,11 @@ int pcg_solve_resident(Context* c, const double4_32a* d_rhs, double rel_tol, int
 // nvec right-hand sides of every RVE of a batch: w = v + K^-1 b per RVE
 int macro_solve_resident(Context* c, int precision, int nvec, const double4_32a* d_b, const double4_32a* d_v,
                          double4_32a* d_w, double rel_tol, int max_it, int precond, int* iters);
+// one launch per solve for whole meshes above the resident capacity (FP32)
+int hybrid_plan(Context* c, bool* fits);
+int hybrid_solve(Context* c, const double4_32a* d_rhs, double rel_tol, int max_it, int precond, int* iters,
+                 double* rel_res);
+void hybrid_reset(Context* c);
 void resident_reset(Context* c);
 void resident_drop_batch(Context* c);
 void resident_destroy(Context* c);
