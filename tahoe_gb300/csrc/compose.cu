@@ -203,15 +203,15 @@ void free_templates(Context* c) {
     delete t;
   }
   c->templates.clear();
-  for (TplGeoPool* p : {&c->tpl_geo_ff, &c->tpl_geo64}) {
+  for (TplGeoPool* p : {&c->tpl_geo_ff, &c->tpl_geo64, &c->tpl_geo_jac}) {
     if (p->d) cudaFreeAsync(p->d, c->stream);
     *p = TplGeoPool{};
   }
   c->tpl_elems = 0;
 }
 
-// The geometry planes of every resident template in one pool (25 planes of
-// 8 points per template element), rebuilt when templates were added since;
+// The geometry planes of every resident template in one pool (8 points
+// per template element), rebuilt when templates were added since;
 // the templates' pool offsets never change.  Without room for it the pool
 // stays empty and batch meshes form their own planes.
 template <typename G>
@@ -222,7 +222,7 @@ int template_geometry_pool(Context* c, TplGeoPool& pool) {
   pool = TplGeoPool{};
   const long long elems = c->tpl_elems;
   G* g = nullptr;
-  if (elems <= 0 || cudaMallocAsync((void**)&g, sizeof(G) * (size_t)elems * 8 * kGeoPlanes, c->stream) != cudaSuccess) {
+  if (elems <= 0 || cudaMallocAsync((void**)&g, sizeof(G) * (size_t)elems * 8 * geo_planes<G>(), c->stream) != cudaSuccess) {
     cudaGetLastError();
     return TG_OK;
   }
@@ -241,6 +241,7 @@ int template_geometry_pool(Context* c, TplGeoPool& pool) {
 }
 template int template_geometry_pool<float2>(Context*, TplGeoPool&);
 template int template_geometry_pool<double>(Context*, TplGeoPool&);
+template int template_geometry_pool<JacPlane>(Context*, TplGeoPool&);
 
 // A template's resident rows and their split for one precision, kept with the
 // template: every batch composed from it uses them.

@@ -1,6 +1,7 @@
 // Element group kernels of the hex8 implicit path on sm_103a.
 //
-//  * residual_kernel  (FP64): one thread per Gauss point, 8 lanes per element.
+//  * residual_kernel  (FP64; total-Lagrangian Simo groups: residual_tl.cu): one
+//    thread per Gauss point, 8 lanes per element.
 //    Kinematics, material stress (with J2 return mapping and history writes)
 //    and the element internal force, reduced over the 8 points with an
 //    in-register shuffle reduce-scatter so lane a ends with node a's force.
@@ -880,7 +881,7 @@ namespace {
 template <typename G>
 int geometry_planes(Context* c, G*& slot) {
   if (slot) return TG_OK;
-  const size_t n = (size_t)c->nel * 8 * kGeoPlanes;
+  const size_t n = (size_t)c->nel * 8 * geo_planes<G>();
   G* g = nullptr;
   if (cudaMallocAsync((void**)&g, n * sizeof(G), c->stream) == cudaSuccess &&
       cudaStreamSynchronize(c->stream) == cudaSuccess) {
@@ -894,9 +895,11 @@ int geometry_planes(Context* c, G*& slot) {
   return TG_OK;
 }
 
-// The double-float residual covers the total-Lagrangian Simo group (every
-// block Simo); the other formulations and materials keep the FP64 kernel.
-bool ff_residual_applies(const Context* c) {
+// The double-float residual and the FP64 one of residual_tl.cu cover the
+// total-Lagrangian Simo group (every block Simo); the other formulations and
+// materials, the output pass and meshes without room for the planes keep
+// residual_kernel.
+bool tl_simo(const Context* c) {
   if (c->mats.formulation != TG_TOTAL_LAGRANGIAN || c->nel <= 0) return false;
   const int nb = c->have_blocks ? c->mats.nblocks : 1;
   for (int b = 0; b < nb; ++b)
@@ -905,7 +908,7 @@ bool ff_residual_applies(const Context* c) {
 }
 
 int residual_impl(Context* c, int commit_state, double* d_ip_sig = nullptr, int arith = kResidualFP64) {
-  if (arith == kResidualDoubleFloat && !d_ip_sig && ff_residual_applies(c)) {
+  if (arith == kResidualDoubleFloat && !d_ip_sig && tl_simo(c)) {
     if (c->composed && c->d_elem_src) {
       // a batch mesh reads its templates' planes
       const int s = template_geometry_pool<float2>(c, c->tpl_geo_ff);
@@ -916,6 +919,17 @@ int residual_impl(Context* c, int commit_state, double* d_ip_sig = nullptr, int 
     const int s = geometry_planes(c, c->d_geo_ff);
     if (s) return s;
     if (c->d_geo_ff) return launch_residual_ff(c, c->d_geo_ff, nullptr, (long long)c->nel * 8);
+  }
+  if (!d_ip_sig && tl_simo(c)) {
+    if (c->composed && c->d_elem_src) {
+      const int s = template_geometry_pool<JacPlane>(c, c->tpl_geo_jac);
+      if (s) return s;
+      if (c->tpl_geo_jac.d)
+        return launch_residual_tl(c, (const JacPlane*)c->tpl_geo_jac.d, c->d_elem_src, c->tpl_geo_jac.elems * 8);
+    }
+    const int s = geometry_planes(c, c->d_geo_jac);
+    if (s) return s;
+    if (c->d_geo_jac) return launch_residual_tl(c, c->d_geo_jac, nullptr, (long long)c->nel * 8);
   }
   // a batch mesh reads its templates' planes; without room for the planes
   // the kernel forms the gradients itself (bitwise the same values)

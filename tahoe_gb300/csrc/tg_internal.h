@@ -74,7 +74,13 @@ struct ResidScalars {
 struct HybState;      // plan and buffers of the hybrid PCG (hybridpcg.cu)
 struct ResState;      // plans and buffers of the resident PCG (respcg.cuh)
 struct MeshTemplate;  // a resident template mesh (compose.cu)
-// geometry planes (25 planes of 8 points per element) of every resident
+// a value of the total-Lagrangian FP64 residual's planes: per point the scaled
+// inverse Jacobian (9) and w det J
+struct JacPlane {
+  double v;
+};
+
+// geometry planes (8 points per element) of every resident
 // template: the element-major offsets are the templates' pool offsets
 struct TplGeoPool {
   void* d = nullptr;
@@ -265,6 +271,7 @@ struct Context {
   float* d_minv32 = nullptr;    // 18*nnd: Jacobi then block-Jacobi
   double* d_minv64 = nullptr;
   double* d_geo = nullptr;      // 25 planes over nel*8 points: dN/dX (3x8), w det J (residual)
+  JacPlane* d_geo_jac = nullptr;  // 10 planes, for the total-Lagrangian Simo residual in FP64
   float2* d_geo_ff = nullptr;   // the same planes as double-floats (hi, lo), for the double-float residual
   int* d_elem_src = nullptr;    // composed mesh: every element's element in the template geometry pool
   double* d_xyz = nullptr;      // nnd*3: staging of caller (x, y, z) nodal arrays
@@ -338,7 +345,7 @@ struct Context {
   // geometry planes of every resident template, one pool per arithmetic
   // (a composed mesh's elements share their template's planes: the batch
   // mesh copies the template's coordinates and connectivity verbatim)
-  TplGeoPool tpl_geo_ff, tpl_geo64;
+  TplGeoPool tpl_geo_ff, tpl_geo64, tpl_geo_jac;
   long long tpl_elems = 0;      // elements of every template added (pool offsets, append-only)
   bool composed = false;           // mesh built by tg_mesh_compose (host copies on demand)
   bool inst_segments = false;      // its RVEs are its instances (no other partition was set)
@@ -430,11 +437,21 @@ void sym_free(Context* c);
 // double-float, everything else FP64.
 enum : int { kResidualFP64 = 0, kResidualDoubleFloat = 1 };
 constexpr int kGeoPlanes = 25;  // per point: dN_a/dX_l (24), w det J
+template <typename G>
+constexpr int geo_planes() {
+  return kGeoPlanes;
+}
+template <>
+constexpr int geo_planes<JacPlane>() {
+  return 10;
+}
 int launch_residual(Context* c, int arith = kResidualFP64);  // fint per element + gather + norm
 // the total-Lagrangian Simo element forces in double-float (residual_ff.cu)
 // src: each element's element in the planes (nullptr: the element itself);
 // gstride: points per plane
 int launch_residual_ff(Context* c, const float2* d_geo_ff, const int* src, long long gstride);
+// the same in FP64 (residual_tl.cu)
+int launch_residual_tl(Context* c, const JacPlane* geo, const int* src, long long gstride);
 // the template geometry pool of one arithmetic (G float2: double-float,
 // double: FP64), built for every resident template (compose.cu)
 template <typename G>
@@ -442,6 +459,9 @@ int template_geometry_pool(Context* c, TplGeoPool& pool);
 template <typename G>
 int launch_geometry(Context* c, const double* X, int nnd, const int* conn, int nel, G* geo, long long stride,
                     long long off);
+template <>
+int launch_geometry<JacPlane>(Context* c, const double* X, int nnd, const int* conn, int nel, JacPlane* geo,
+                              long long stride, long long off);
 int launch_tangent(Context* c, int precision);   // Ke per element
 // the same for moduli of the isotropic form (tangent_iso.cu)
 bool tangent_iso_applies(const Context* c, int precision);
