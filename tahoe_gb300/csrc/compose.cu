@@ -274,15 +274,14 @@ int template_resident(Context* c, int tpl, int precision, ResPlan& P, bool& fits
     t->res_built = true;
   }
   if (t->res_state[p] == 0) {
-    size_t cap = 0;
-    int cluster = 1;
-    int s = resident_limits(c, precision, &cap, &cluster);
+    ResLimits limits;
+    int s = resident_limits(c, precision, &limits);
     if (s) return s;
     ResPlan& Q = t->res_plan[p];
     Q = ResPlan{};
     if (t->res_rows.act_node.empty()) {
       t->res_state[p] = 1;  // nothing to solve
-    } else if (resident_plan(t->res_rows, p ? 4 : 8, c->num_sms, cap, cluster, false, Q)) {
+    } else if (resident_plan(t->res_rows, p ? 4 : 8, c->num_sms, limits, false, Q)) {
       ResImage img;
       const size_t at = img.split_at(Q);
       int* d = nullptr;

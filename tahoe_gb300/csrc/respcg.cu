@@ -55,13 +55,13 @@ namespace tg {
 namespace {
 
 // One CTA's part of one solve.
-template <typename T, bool GRID, bool BLK>
+template <typename T, bool GRID, bool BLK, int NS>
 __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResItem& I, int item, int rank,
                                                unsigned char* smem, ResShared<T>& sh) {
   using V = typename Vec4<T>::type;
   using Shape = ResShape<T>;
   constexpr bool F32 = sizeof(T) == 4;
-  constexpr int NS = Shape::slots, RB = Shape::reg, OFF = Shape::off, RA = RB > 0 ? RB : 1, NM = BLK ? 3 : 1;
+  constexpr int RB = Shape::reg, OFF = Shape::off, RA = RB > 0 ? RB : 1, NM = BLK ? 3 : 1;
   const ResPlanDev P = A.plans[I.plan];
   const int k = P.k;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, c = lane & 3, q0 = lane & ~3;
@@ -117,8 +117,8 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
   uint16_t* cols = reinterpret_cast<uint16_t*>(vals + (size_t)vsteps * 9 * 32);
   uint4* inbox = GRID ? A.ll + I.ll : nullptr;                         // partial sums
   uint4* urow = GRID ? inbox + 4 * (size_t)min(k, kResCopies) * k : nullptr;  // rows' vectors
-  // columns of this warp's quarter: two chunks of 64
-  const unsigned tm = F32 ? sh.tmem + ((unsigned)(warp & 3) << 21) + (unsigned)(warp >> 2) * 128u : 0u;
+  // columns of this warp's quarter: two chunks of 64 (FP64: one of 126)
+  const unsigned tm = sh.tmem + ((unsigned)(warp & 3) << 21) + (unsigned)(warp >> 2) * 128u;
   const long long at0 = (long long)I.vec * A.nnd + I.node_off;  // of this right-hand side
   if (threadIdx.x == 0) sh.abort_flag = 0;
   if (!GRID && k > 1) {
@@ -203,7 +203,25 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
           tmem_st9(tm + (unsigned)(q - 1) * 64u + 9u * (unsigned)t, acc);
         }
     }
-    const int off = q == 0 ? RB : q < OFF ? Shape::tm : 0;
+    if constexpr (!F32) {
+      if (q == 0 && nw == Shape::warps)
+        for (int t = 0; t < Shape::tm; ++t) {
+          T acc[9];
+#pragma unroll
+          for (int e = 0; e < 9; ++e) acc[e] = T(0);
+          if (t < nst) block(t, acc);
+          float h[18];
+#pragma unroll
+          for (int e = 0; e < 9; ++e) {
+            h[2 * e] = __int_as_float(__double2loint(acc[e]));
+            h[2 * e + 1] = __int_as_float(__double2hiint(acc[e]));
+          }
+          __syncwarp();
+          tmem_st9(tm + 18u * (unsigned)t, h);
+          tmem_st9(tm + 18u * (unsigned)t + 9u, h + 9);
+        }
+    }
+    const int off = F32 ? (q == 0 ? RB : q < OFF ? Shape::tm : 0) : q == 0 && nw == Shape::warps ? Shape::tm : 0;
     for (int t = off; t < nst; ++t) {
       T acc[9];
       block(t, acc);
@@ -237,7 +255,7 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
       pr[q] = sr[q] = xr[q] = T(0);
     }
   }
-  if constexpr (F32) tmem_wait_st();
+  if (F32 || nw == Shape::warps) tmem_wait_st();
   // M^-1 r of a row's component (whole warps; zero for a warp without a chunk)
   auto precond = [&](int q, T rq) {
     const bool on = warp + q * nw < nch;
@@ -425,6 +443,23 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
           }
         }
       }
+      if constexpr (!F32) {
+        if (q == 0 && nw == Shape::warps && nst > 0) {
+          const uint4 g = *cg;
+#pragma unroll
+          for (int t = 0; t < Shape::tm; ++t)
+            if (t < 4 || nst > 4) {
+              unsigned b[18];
+              __syncwarp();
+              tmem_ld18(tm + 18u * (unsigned)t, b);
+              const V uj = uw[index(g, t)];
+              tmem_wait_ld();
+              auto f = [&](int e) { return __hiloint2double((int)b[2 * e + 1], (int)b[2 * e]); };
+              fma9(f(0), f(1), f(2), f(3), f(4), f(5), f(6), f(7), f(8), uj);
+            }
+          t0 = Shape::tm;
+        }
+      }
       for (; t0 < nst; t0 = (t0 | 7) + 1) {
         const uint4 g = cg[(t0 >> 3) * 32];
         const int e = min(nst, (t0 | 7) + 1);
@@ -558,10 +593,11 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
 }
 
 // Tensor memory of a CTA with all its warps: such a CTA has the SM to itself
-// (512 threads at 128 registers), so the allocation never waits for another.
+// (its launch asks for more than half the shared memory), so the allocation
+// never waits for another.
 template <typename T>
 __device__ __forceinline__ bool tmem_begin(ResShared<T>& sh) {
-  const bool use = sizeof(T) == 4 && blockDim.x == ResShape<T>::warps * 32;
+  const bool use = blockDim.x == ResShape<T>::warps * 32;
   if (use && threadIdx.x < 32) tmem_alloc(&sh.tmem);
   __syncthreads();
   return use;
@@ -572,29 +608,43 @@ __device__ __forceinline__ void tmem_end(ResShared<T>& sh, bool use) {
   if (use && threadIdx.x < 32) tmem_free(sh.tmem);
 }
 
-template <typename T, bool BLK>
+template <typename T, bool BLK, int NS>
 __global__ void __launch_bounds__(ResShape<T>::warps * 32, 1) resident_cluster_kernel(ResArgs<T> A) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ ResShared<T> sh;
   const int item = blockIdx.x / A.k, rank = blockIdx.x % A.k;
   const bool tmem = tmem_begin(sh);
-  resident_solve<T, false, BLK>(A, A.items[item], item, rank, smem, sh);
+  resident_solve<T, false, BLK, NS>(A, A.items[item], item, rank, smem, sh);
   tmem_end(sh, tmem);
 }
 
-template <typename T, bool BLK>
+template <typename T, bool BLK, int NS>
 __global__ void __launch_bounds__(ResShape<T>::warps * 32, 1) resident_grid_kernel(ResArgs<T> A) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ ResShared<T> sh;
   const bool tmem = tmem_begin(sh);
   const int groups = gridDim.x / A.k, rank = blockIdx.x % A.k;
   for (int item = blockIdx.x / A.k; item < A.count; item += groups) {
-    resident_solve<T, true, BLK>(A, A.items[item], item, rank, smem, sh);
+    resident_solve<T, true, BLK, NS>(A, A.items[item], item, rank, smem, sh);
     const bool stop = sh.abort_flag != 0;
     __syncthreads();
     if (stop) break;  // a wait ran out: nothing more is awaited
   }
   tmem_end(sh, tmem);
+}
+
+// The kernel of a launch class.  FP64 has one for parts of at most a chunk a
+// warp (NS = 1): the second chunk's code costs a single solve of 4,000 rows 7%.
+template <typename T>
+const void* resident_kernel(bool grid, bool blk, bool one) {
+  constexpr int N = ResShape<T>::slots, L = sizeof(T) == 8 ? 1 : N;
+  if (one)
+    return grid ? (blk ? (const void*)resident_grid_kernel<T, true, L> : (const void*)resident_grid_kernel<T, false, L>)
+                : (blk ? (const void*)resident_cluster_kernel<T, true, L>
+                       : (const void*)resident_cluster_kernel<T, false, L>);
+  return grid ? (blk ? (const void*)resident_grid_kernel<T, true, N> : (const void*)resident_grid_kernel<T, false, N>)
+              : (blk ? (const void*)resident_cluster_kernel<T, true, N>
+                     : (const void*)resident_cluster_kernel<T, false, N>);
 }
 
 // The rows of a whole mesh on the device (a mesh of 50,000 nodes took 17 ms on
@@ -674,34 +724,30 @@ __global__ void resident_slots_kernel(long long n, const int* __restrict__ blk, 
 
 // ---- planning ---------------------------------------------------------------
 
-// Dynamic shared memory of one CTA and the largest cluster that can run with it.
+// Dynamic shared memory of one CTA, the largest cluster that can run with it,
+// and for every cluster size the largest with as many at a time on the chip.
 template <typename T>
-int limits_t(Context* c, size_t* cap, int* cluster) {
+int limits_t(Context* c, ResLimits* L) {
   int optin = 0;
   cudaFuncAttributes fa;
   if (!ok(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device), "attribute"))
     return TG_ERR_CUDA;
   size_t smem = (size_t)optin;
-  for (const void* fn : {reinterpret_cast<const void*>(resident_cluster_kernel<T, false>),
-                         reinterpret_cast<const void*>(resident_cluster_kernel<T, true>),
-                         reinterpret_cast<const void*>(resident_grid_kernel<T, false>),
-                         reinterpret_cast<const void*>(resident_grid_kernel<T, true>)}) {
+  for (int q = 0; q < 8; ++q) {
+    const void* fn = resident_kernel<T>(q & 1, q & 2, q & 4);
     if (!ok(c, cudaFuncGetAttributes(&fa, fn), "function attributes")) return TG_ERR_CUDA;
     smem = std::min(smem, (size_t)optin - fa.sharedSizeBytes);
     // one value for every caller: other contexts may configure and launch it
     if (!ok(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes),
-            "smem attribute"))
+            "smem attribute") ||
+        (!(q & 1) &&
+         !ok(c, cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cluster attribute")))
       return TG_ERR_CUDA;
   }
-  *cap = smem;
-  *cluster = 1;
-  const void* fn = reinterpret_cast<const void*>(resident_cluster_kernel<T, true>);
-  if (!ok(c, cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cluster attribute") ||
-      !ok(c, cudaFuncSetAttribute(reinterpret_cast<const void*>(resident_cluster_kernel<T, false>),
-                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
-          "cluster attribute"))
-    return TG_ERR_CUDA;
-  for (int k = kResClusterMax; k > 1; k /= 2) {
+  L->smem = smem;
+  L->cluster = 1;
+  int many[kResClusterMax + 1] = {};
+  for (int k = 1; k <= kResClusterMax; ++k) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(k);
     cfg.blockDim = dim3(ResShape<T>::warps * 32);
@@ -712,12 +758,15 @@ int limits_t(Context* c, size_t* cap, int* cluster) {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n > 0) {
-      *cluster = k;
-      break;
-    }
-    cudaGetLastError();
+    if (cudaOccupancyMaxActiveClusters(&many[k], resident_kernel<T>(false, true, false), &cfg) == cudaSuccess &&
+        many[k] > 0)
+      L->cluster = (k & (k - 1)) == 0 ? k : L->cluster;
+    else
+      cudaGetLastError();
+  }
+  for (int k = 1; k <= kResClusterMax; ++k) {
+    L->widest[k] = k;
+    for (int j = k + 1; j <= L->cluster && many[k] > 0 && many[j] == many[k]; ++j) L->widest[k] = j;
   }
   return TG_OK;
 }
@@ -780,7 +829,8 @@ void resident_rows(int n0, int n1, const int* rowptr, const int* col, const uint
 namespace {
 
 // Bytes of one part with nw warps: the window, FP32's vectors and
-// preconditioner, the values outside registers and tensor memory (res_off_steps), the columns in groups of eight steps.
+// preconditioner, the values outside registers and tensor memory
+// (res_off_steps), the columns in groups of eight steps.
 size_t part_bytes(const ResRows& R, int a, int b, int elem, int nw, int* lo, int* hi) {
   int l = R.chunk_lo[a], h = R.chunk_hi[a];
   const int state = elem == 4 ? ResShape<float>::state : ResShape<double>::state;
@@ -831,6 +881,7 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
   if (most > warps * slots) return false;
   // one chunk per warp while there are warps for it
   P.warps = std::min(warps, (most + 3) / 4 * 4);
+  P.one = elem == 8 && most <= P.warps;
   for (int q = 0; q < k; ++q) {
     const int a = P.part_chunk[q], b = P.part_chunk[q + 1];
     int lo, hi;
@@ -856,10 +907,13 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
 }  // namespace
 
 // A split of the rows over CTAs.  A solve of a batch takes the fewest CTAs
-// that hold it (every SM has another RVE to solve); a solve alone spreads
+// that hold it (every SM has another RVE to solve), in FP64 as many more as
+// leave the number of clusters that run at once the same; a solve alone spreads
 // over the chip.  Up to the cluster limit the CTAs are one cluster, above it
 // (grid) CTAs of a cooperative launch.
-bool resident_plan(const ResRows& R, int elem, int num_sms, size_t cap, int max_cluster, bool alone, ResPlan& P) {
+bool resident_plan(const ResRows& R, int elem, int num_sms, const ResLimits& L, bool alone, ResPlan& P) {
+  const size_t cap = L.smem;
+  const int max_cluster = L.cluster;
   const int nch = (int)R.chunk_lo.size();
   P.rows = R.rows;
   P.nchunks = nch;
@@ -877,6 +931,13 @@ bool resident_plan(const ResRows& R, int elem, int num_sms, size_t cap, int max_
     const int few = elem == 4 ? 24 : 4;
     P.grid = P.grid || (nch + max_cluster - 1) / max_cluster > few;
     const int k = std::max(kmin, std::min(nch, P.grid ? num_sms : max_cluster));
+    if (k != kmin && !split_parts(R, k, elem, cap, P) && !split_parts(R, kmin, elem, cap, P)) return false;
+  } else if (!P.grid && elem == 8) {
+    // the chip holds 15 clusters of 7, of 8 and of 9: in FP64, where a CTA's
+    // time is that of its chunks, the largest costs nothing (48 RVEs with nine
+    // solves each 31.2 -> 29.9 ms); FP32's time is the exchanges' (64 RVEs
+    // 6.95 -> 7.18 ms)
+    const int k = std::min(nch, L.widest[kmin]);
     if (k != kmin && !split_parts(R, k, elem, cap, P) && !split_parts(R, kmin, elem, cap, P)) return false;
   }
   return true;
@@ -911,16 +972,15 @@ void resident_bind_split(ResPlanDev& D, const int* base, size_t at, const ResPla
   D.nchunks = P.nchunks;
 }
 
-int resident_limits(Context* c, int precision, size_t* smem, int* cluster) {
+int resident_limits(Context* c, int precision, ResLimits* limits) {
   ResState& S = *c->res;
   const int p = precision == TG_MIXED ? 1 : 0;
   if (!S.limits_known[p]) {
-    const int s = p ? limits_t<float>(c, &S.smem[p], &S.cluster[p]) : limits_t<double>(c, &S.smem[p], &S.cluster[p]);
+    const int s = p ? limits_t<float>(c, &S.limits[p]) : limits_t<double>(c, &S.limits[p]);
     if (s) return s;
     S.limits_known[p] = true;
   }
-  *smem = S.smem[p];
-  *cluster = S.cluster[p];
+  *limits = S.limits[p];
   return TG_OK;
 }
 
@@ -1032,9 +1092,8 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
   M = ResMode{};
   M.state = -1;
   const int elem = precision == TG_MIXED ? 4 : 8;
-  size_t cap = 0;
-  int cluster = 1;
-  int s = resident_limits(c, precision, &cap, &cluster);
+  ResLimits limits;
+  int s = resident_limits(c, precision, &limits);
   if (s) return s;
   const int nseg = batch ? c->nseg : 1;
   if (batch && c->inst_segments) {
@@ -1063,7 +1122,7 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
     ResPlan P;
     s = rows_of_mesh(c, R, P.dev);
     if (s) return s;
-    if (!resident_plan(R, elem, c->num_sms, cap, cluster, true, P)) return TG_OK;
+    if (!resident_plan(R, elem, c->num_sms, limits, true, P)) return TG_OK;
     ResImage img;
     const size_t at = img.split_at(P);
     int* d = nullptr;
@@ -1088,7 +1147,7 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
       const int n0 = c->h_seg_node[i], n1 = c->h_seg_node[i + 1];
       resident_rows(n0, n1, c->h_rowptr.data(), c->h_col.data(), mask.data(), rows[i]);
       ResPlan P;
-      if (!rows[i].act_node.empty() && !resident_plan(rows[i], elem, c->num_sms, cap, cluster, false, P)) return TG_OK;
+      if (!rows[i].act_node.empty() && !resident_plan(rows[i], elem, c->num_sms, limits, false, P)) return TG_OK;
       at_rows[i] = img.rows_at(rows[i]);
       at_split[i] = img.split_at(P);
       M.plans.push_back(P);
@@ -1157,7 +1216,7 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
   const int nseg = (int)act.size();
   // launch classes by form, CTAs, warps and shared memory, the largest first
   struct Class {
-    bool grid;
+    bool grid, one;
     int k, warps;
     size_t smem;
     std::vector<int> seg;
@@ -1167,8 +1226,9 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
     const ResPlan& P = M.plans[M.plan_of[i]];
     if (!act[i] || P.rows == 0) continue;
     const long long b = (long long)((P.smem + 16383) / 16384);
-    Class& C = cls[{P.grid ? 0 : 1, -(long long)P.k, -P.warps, -b}];
+    Class& C = cls[{P.grid ? 0 : 1, -(long long)P.k, -P.warps, P.one ? 1 : 0, -b}];
     C.grid = P.grid;
+    C.one = P.one;
     C.k = P.k;
     C.warps = P.warps;
     C.smem = std::max(C.smem, P.smem);
@@ -1239,8 +1299,10 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
   }
   size_t first = 0;
   int q = 0;
-  for (const auto& e : cls) {
-    const Class& C = e.second;
+  for (auto& e : cls) {
+    Class& C = e.second;
+    // a CTA that allocates tensor memory: alone on its SM
+    if (C.warps == ResShape<T>::warps) C.smem = std::max(C.smem, (size_t)116 << 10);
     const size_t solves = C.seg.size() * (size_t)nvec;
     ResArgs<T> B = A;
     B.items = S.d_items + first;
@@ -1267,9 +1329,9 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
     cfg.attrs = at;
     cfg.numAttrs = 1;
     c->launches++;
-    auto* fn = C.grid ? (blk ? resident_grid_kernel<T, true> : resident_grid_kernel<T, false>)
-                      : (blk ? resident_cluster_kernel<T, true> : resident_cluster_kernel<T, false>);
-    if (!ok(c, cudaLaunchKernelEx(&cfg, fn, B), C.grid ? "resident_grid_kernel" : "resident_cluster_kernel"))
+    void* args[] = {&B};
+    if (!ok(c, cudaLaunchKernelExC(&cfg, resident_kernel<T>(C.grid, blk, C.one), args),
+            C.grid ? "resident_grid_kernel" : "resident_cluster_kernel"))
       return TG_ERR_CUDA;
     ++q;
   }

@@ -45,11 +45,20 @@ struct ResRows {
   std::vector<int> act_node, blk, col, chunk_step, chunk_lo, chunk_hi;
 };
 
+// What a CTA and the chip hold: dynamic shared memory, the largest cluster, and
+// for every cluster size the largest with as many at a time.
+struct ResLimits {
+  size_t smem = 0;
+  int cluster = 1;
+  int widest[17] = {};
+};
+
 // A split of them over CTAs for one precision (host) and its device copy.
 struct ResPlan {
   int rows = 0, nchunks = 0, k = 0, warps = 0;  // warps: of every CTA
   size_t smem = 0;                              // the largest part's bytes
   bool grid = false;
+  bool one = false;                             // no warp has more than one chunk
   std::vector<int> part_chunk;
   std::vector<int4> part_win;
   ResPlanDev dev{};
@@ -76,12 +85,11 @@ struct ResState {
   cudaStream_t aux[kResAux] = {};
   cudaEvent_t fork = nullptr, join[kResAux] = {};
   bool limits_known[2] = {false, false};
-  size_t smem[2] = {0, 0};
-  int cluster[2] = {1, 1};
+  ResLimits limits[2];
 };
 
 void resident_rows(int n0, int n1, const int* rowptr, const int* col, const uint8_t* mask, ResRows& R);
-bool resident_plan(const ResRows& R, int elem, int num_sms, size_t cap, int max_cluster, bool alone, ResPlan& P);
+bool resident_plan(const ResRows& R, int elem, int num_sms, const ResLimits& L, bool alone, ResPlan& P);
 
 // The device copy of a template's rows and its plan for one precision
 // (compose.cu), built on first use.
@@ -96,6 +104,6 @@ struct ResImage {
 void resident_bind_rows(ResPlanDev& D, const int* base, size_t at, const ResRows& R);
 void resident_bind_split(ResPlanDev& D, const int* base, size_t at, const ResPlan& P);
 int resident_slots(Context* c, long long n, const int* d_blk, const int* d_cptr, int2* d_slot);
-int resident_limits(Context* c, int precision, size_t* smem, int* cluster);
+int resident_limits(Context* c, int precision, ResLimits* limits);
 
 }  // namespace tg

@@ -30,7 +30,13 @@ constexpr int kResPollLimit = 1 << 21;  // polls of one exchange word before the
 // from shared memory).  Fewer CTAs a solve also means more solves at once: a
 // chip runs 46 clusters of 3 CTAs, 28 of 5, 15 of 7 to 9, 8 of 11 or 12.
 // FP64 runs at the rate of the FP64 pipe (one warp instruction per 64 cycles
-// and scheduler), not of the storage: shared memory alone.
+// and scheduler), not of the storage.  A CTA of 16 warps keeps the first chunk
+// of each warp in tensor memory and a second in shared memory where there is
+// room: 29 chunks where shared memory alone held 13, so a solve of a batch
+// takes half the CTAs, the 6,000 cycles of exchange and sums an iteration
+// stand beside twice the product, and clusters of 6 fill the chip where
+// clusters of 13 leave 61 of 152 SMs out.  (Smaller CTAs, several to an SM,
+// allocate no tensor memory.)
 template <typename T>
 struct ResShape;
 template <>
@@ -39,11 +45,12 @@ struct ResShape<float> {
 };
 template <>
 struct ResShape<double> {
-  static constexpr int warps = 16, slots = 1, reg = 0, tm = 0, off = 0, state = 0;
+  static constexpr int warps = 16, slots = 2, reg = 0, tm = 7, off = 1, state = 0;
 };
 // steps of chunk i of a part of nw warps that stay out of shared memory
 template <typename T>
 __host__ __device__ constexpr int res_off_steps(int i, int nw) {
+  if (sizeof(T) == 8) return nw == ResShape<T>::warps && i < ResShape<T>::off * nw ? ResShape<T>::tm : 0;
   return i < nw ? ResShape<T>::reg : i < ResShape<T>::off * nw ? ResShape<T>::tm : 0;
 }
 constexpr int kTmemColumns = 512;
