@@ -1,5 +1,5 @@
-// Hybrid PCG, sm_103a: one launch per solve for a mesh above the resident
-// capacity (respcg.cu), FP32 form.
+// Hybrid PCG, sm_103a: one launch per solve for a whole mesh of 20,000 nodes
+// and more, FP32 form (smaller meshes and RVE batches: respcg.cu).
 //
 // The push-storage solve (pcg_cg.cu) streams half the matrix every iteration
 // (174 MB on the 64^3 block) and passes 55 MB of transposed products through

@@ -1474,6 +1474,8 @@ int macro_solve_resident(Context* c, int precision, int nvec, const double4_32a*
 // The default form solves resident where the mesh (every RVE of the batch)
 // fits; the explicit forms of tg_pcg_form and the symmetric format keep their
 // own kernels.
+constexpr int kHybridNodes = 20000;
+
 int resident_active(Context* c, int precision, bool* on) {
   *on = false;
   if (c->cg_push >= 0 || c->pcg_form != 1 || !c->cg_pdl || sym_active(c)) return TG_OK;
@@ -1482,12 +1484,18 @@ int resident_active(Context* c, int precision, bool* on) {
   const bool batch = c->nseg > 0 && c->seg_pcg_mode;
   ResMode& M = c->res->mode[precision == TG_MIXED ? 1 : 0][batch ? 1 : 0];
   if (M.state == 0) {
-    int s = plan_mode(c, precision, batch, M);
-    if (!s && M.state < 0 && !batch && precision == TG_MIXED) {
-      bool fits = false;
-      s = hybrid_plan(c, &fits);
-      if (fits) M.state = 2;
-    }
+    // A whole mesh in FP32 above kHybridNodes: the hybrid form, whose compact
+    // parts exchange a fifth of the rows that the grid form's slabs do.  Per
+    // iteration, grid form / hybrid: 3,375 nodes 4.7 / 5.2 us, 9,261 5.2 / 4.4,
+    // 15,625 4.8 / 5.1, 27,360 6.3 / 5.1, 38,475 7.4 / 5.7, 60,025 9.0 / 6.9.
+    // The grid form keeps what the hybrid refuses.
+    int s = TG_OK;
+    bool fits = false;
+    if (!batch && precision == TG_MIXED && c->nnd >= kHybridNodes) s = hybrid_plan(c, &fits);
+    if (!s && fits)
+      M.state = 2;
+    else if (!s)
+      s = plan_mode(c, precision, batch, M);
     if (s) return s;
   }
   *on = M.state > 0;
