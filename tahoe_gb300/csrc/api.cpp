@@ -66,30 +66,14 @@ void free_all(Context* c) {
   if (c->h_pcg) cudaFreeHost(c->h_pcg);
   if (c->h_resid) cudaFreeHost(c->h_resid);
   if (c->h_status) cudaFreeHost(c->h_status);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
+  c->h_stage = nullptr;
   c->h_pcg = nullptr;
   c->h_resid = nullptr;
   c->h_status = nullptr;
 }
 
 int set_device(Context* c) { return ok(c, cudaSetDevice(c->device), "cudaSetDevice") ? TG_OK : TG_ERR_CUDA; }
-
-// read back the device status word and residual norm; clears the status
-int sync_status(Context* c) {
-  if (!ok(c, cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "status"))
-    return TG_ERR_CUDA;
-  if (!ok(c, cudaStreamSynchronize(c->stream), "sync")) return TG_ERR_CUDA;
-  const int st = *c->h_status;
-  if (st) {
-    cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream);
-    if (st & kStatusBadJacobian) {
-      c->err = "non-positive Jacobian determinant";
-      return TG_ERR_BAD_JACOBIAN;
-    }
-    c->err = "non-finite value";
-    return TG_ERR_NAN;
-  }
-  return TG_OK;
-}
 
 bool valid_material(int kind, const double* p, int np, MatParams& m) {
   std::memset(&m, 0, sizeof(m));
@@ -267,7 +251,8 @@ int tg_create(tg_context** out, int device) {
       !ok(c, cudaEventCreateWithFlags(&c->ev_poll[0], cudaEventDisableTiming), "event") ||
       !ok(c, cudaEventCreateWithFlags(&c->ev_poll[1], cudaEventDisableTiming), "event") ||
       !ok(c, cudaMallocHost((void**)&c->h_resid, sizeof(ResidScalars)), "pinned") ||
-      !ok(c, cudaMallocHost((void**)&c->h_status, sizeof(int)), "pinned")) {
+      !ok(c, cudaMallocHost((void**)&c->h_status, sizeof(int)), "pinned") ||
+      !ok(c, cudaMallocHost((void**)&c->h_stage, kStageBytes), "pinned")) {
     free_all(c);
     delete c;
     return TG_ERR_CUDA;
@@ -624,6 +609,13 @@ int tg_pattern_build_host(int nnd, int nel, const int* conn, const int* eqnos, i
 int tg_set_displacement(tg_context* c, const double* u) {
   if (!c || !u || c->nnd <= 0) return TG_ERR_ARG;
   if (set_device(c)) return TG_ERR_CUDA;
+  const size_t bytes = sizeof(double) * 3 * c->nnd;
+  if (bytes <= kStageBytes) {
+    std::memcpy(c->h_stage, u, bytes);
+    const int s = launch_xyz_to_nodal(c, c->h_stage, c->d_u);
+    if (s) return s;
+    return ok(c, cudaStreamSynchronize(c->stream), "sync") ? TG_OK : TG_ERR_CUDA;
+  }
   if (!c->d_xyz && !dalloc(c, &c->d_xyz, (size_t)c->nnd * 3)) return TG_ERR_OOM;
   if (!ok(c, cudaMemcpyAsync(c->d_xyz, u, sizeof(double) * 3 * c->nnd, cudaMemcpyHostToDevice, c->stream), "u"))
     return TG_ERR_CUDA;
@@ -635,6 +627,14 @@ int tg_set_displacement(tg_context* c, const double* u) {
 int tg_get_displacement(tg_context* c, double* u) {
   if (!c || !u || c->nnd <= 0) return TG_ERR_ARG;
   if (set_device(c)) return TG_ERR_CUDA;
+  const size_t bytes = sizeof(double) * 3 * c->nnd;
+  if (bytes <= kStageBytes) {
+    const int s = launch_nodal_to_xyz(c, c->d_u, c->h_stage);
+    if (s) return s;
+    if (!ok(c, cudaStreamSynchronize(c->stream), "sync")) return TG_ERR_CUDA;
+    std::memcpy(u, c->h_stage, bytes);
+    return TG_OK;
+  }
   if (!c->d_xyz && !dalloc(c, &c->d_xyz, (size_t)c->nnd * 3)) return TG_ERR_OOM;
   const int s = launch_nodal_to_xyz(c, c->d_u, c->d_xyz);
   if (s) return s;
@@ -733,10 +733,13 @@ int tg_form_residual_precision(tg_context* c, int precision, double* R_out, doub
   if (set_device(c)) return TG_ERR_CUDA;
   int s = launch_residual(c, precision == TG_MIXED ? kResidualDoubleFloat : kResidualFP64);
   if (s) return s;
-  if (!ok(c, cudaMemcpyAsync(c->h_resid, c->d_resid, sizeof(ResidScalars), cudaMemcpyDeviceToHost, c->stream), "norm"))
-    return TG_ERR_CUDA;
   double* d_eq = nullptr;
-  if (R_out && c->neq > 0) {
+  const size_t bytes = sizeof(double) * c->neq;
+  const bool staged = R_out && bytes <= kStageBytes;
+  if (staged) {
+    s = launch_gather_eq(c, c->d_R, c->h_stage);
+    if (s) return s;
+  } else if (R_out && c->neq > 0) {
     if (!ok(c, cudaMallocAsync((void**)&d_eq, sizeof(double) * c->neq, c->stream), "alloc")) return TG_ERR_OOM;
     s = launch_gather_eq(c, c->d_R, d_eq);
     if (!s && !ok(c, cudaMemcpyAsync(R_out, d_eq, sizeof(double) * c->neq, cudaMemcpyDeviceToHost, c->stream), "R"))
@@ -744,7 +747,8 @@ int tg_form_residual_precision(tg_context* c, int precision, double* R_out, doub
     cudaFreeAsync(d_eq, c->stream);
     if (s) return s;
   }
-  s = sync_status(c);
+  s = residual_status(c);
+  if (staged && s != TG_ERR_CUDA) std::memcpy(R_out, c->h_stage, bytes);
   if (s) return s;
   const double n2 = c->h_resid->norm2;
   if (!std::isfinite(n2)) {

@@ -29,9 +29,16 @@ bool copy_sync(Context* c, void* dst, const void* src, size_t bytes, cudaMemcpyK
 }
 
 int check_status(Context* c) {
-  if (!ok(c, cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "status") ||
-      !ok(c, cudaStreamSynchronize(c->stream), "sync"))
+  if (!ok(c, cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream), "status"))
     return TG_ERR_CUDA;
+  return residual_status(c);
+}
+}  // namespace
+
+// After a residual, whose gather wrote the host mirrors of the norm and the
+// status word: waits for it and returns the status (cleared if set).
+int residual_status(Context* c) {
+  if (!ok(c, cudaStreamSynchronize(c->stream), "sync")) return TG_ERR_CUDA;
   const int st = *c->h_status;
   if (!st) return TG_OK;
   cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream);
@@ -44,6 +51,8 @@ int check_status(Context* c) {
   return TG_ERR_NAN;
 }
 
+namespace {
+
 // arithmetic of the residuals a Newton driver forms: the mixed-precision
 // form's are double-float (48 significant bits, on the FP32 pipe), the FP64
 // form's are FP64
@@ -54,10 +63,7 @@ int residual_arith(const tg_newton_params* P) {
 // residual on the device; returns its norm
 int residual_norm(Context* c, double* norm, int arith) {
   int s = launch_residual(c, arith);
-  if (s) return s;
-  if (!ok(c, cudaMemcpyAsync(c->h_resid, c->d_resid, sizeof(ResidScalars), cudaMemcpyDeviceToHost, c->stream), "norm"))
-    return TG_ERR_CUDA;
-  s = check_status(c);
+  if (!s) s = residual_status(c);
   if (s) return s;
   const double n2 = c->h_resid->norm2;
   if (!std::isfinite(n2)) {
@@ -542,7 +548,7 @@ int predict(tg_context* c, int n, const int* idx, const double* val, const doubl
   if (pcg_iterations) *pcg_iterations = 0;
   // R(u_old) without committing history, tangent at u_old
   int s = launch_residual_nocommit(c, residual_arith(P));
-  if (!s) s = check_status(c);
+  if (!s) s = residual_status(c);
   if (!s) s = form_tangent(c, P->precision);
   if (s) return s;
   double4_32a *d_old = nullptr, *d_v = nullptr;

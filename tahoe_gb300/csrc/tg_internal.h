@@ -319,6 +319,7 @@ struct Context {
   cudaEvent_t ev_poll[2] = {nullptr, nullptr};  // arrival of each mirror's copy
   ResidScalars* h_resid = nullptr;   // pinned mirror
   int* h_status = nullptr;           // pinned mirror
+  double* h_stage = nullptr;         // pinned, kStageBytes: small vectors between caller and device
   double4_32a* d_du_last = nullptr;      // FP64 update (nnd)
   bool have_du = false;
 
@@ -552,6 +553,7 @@ size_t pcg_scratch_bytes(const Context* c);
 int pcg_solve_scratch(Context* c, const double* d_rhs_eq, double* d_du_eq, unsigned char* scratch, double rel_tol,
                       int max_it, int precond, int* iters, double* rel_res);
 int launch_residual_nocommit(Context* c, int arith = kResidualFP64);
+int residual_status(Context* c);  // after either: waits, status (newton.cpp)
 // output pass (no history written): per point the Cauchy stress and the J2
 // material output (alpha, von Mises, pressure) into d_ip_sig (nel*8*9), the
 // extrapolated, element-averaged nodal values into d_out (nnd*9)
@@ -560,6 +562,11 @@ int launch_nodal_stress(Context* c, double* d_ip_sig, double* d_out);
 // accumulation; with zero_base, rhs = -K v
 int launch_lift_rhs(Context* c, const double4_32a* d_v, double4_32a* d_rhs, bool zero_base = false, int nvec = 1);
 int launch_diff(Context* c, const double4_32a* a, const double4_32a* b, double4_32a* out);
+// Vectors up to this size pass between the caller's memory and the kernels
+// through pinned memory that the kernels read and write themselves: a pageable
+// copy costs 10 us before its first byte and 22 us a megabyte, the host's own
+// copy about 100 us a megabyte.
+constexpr size_t kStageBytes = 128 << 10;
 int launch_gather_eq(Context* c, const double4_32a* d_nodal, double* d_eq);
 int launch_xyz_to_nodal(Context* c, const double* d_xyz, double4_32a* d_nodal);  // 3 -> padded 4 per node
 int launch_nodal_to_xyz(Context* c, const double4_32a* d_nodal, double* d_xyz);
