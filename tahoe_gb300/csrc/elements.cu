@@ -10,8 +10,8 @@
 //  * gather_residual_kernel: R = factor*Fext - sum of element forces per node,
 //    in the fixed node->element incidence order (no atomics), fused with the
 //    FP64 norm (SolverT::Residual, SolverT.cpp:848).
-//  * tangent_kernel<T> (B-bar, updated Lagrangian, anisotropic and St.Venant
-//    moduli; the isotropic ones: tangent_iso.cu): 8 elements per CTA.  64 threads stage per-point
+//  * tangent_kernel<T> (B-bar, updated Lagrangian, anisotropic moduli; the
+//    others: tangent_iso.cu, tangent_blocks.cu): 8 elements per CTA.  64 threads stage per-point
 //    gradients, moduli and stress in shared memory; then one thread per
 //    upper node-pair block (36 per element) integrates its 3x3 block of
 //    B^T c B (+ geometric stiffness for TL) over the 8 points.
@@ -1059,6 +1059,8 @@ void launch_tangent_epb(Context* c, int precision) {
 
 int launch_tangent(Context* c, int precision) {
   if (tangent_iso_applies(c, precision)) return launch_tangent_iso(c);
+  // another number of elements per CTA asks for the general kernel
+  if (c->tangent_epb == kTanElems && tangent_blocks_applies(c, precision)) return launch_tangent_blocks(c, precision);
   switch (c->tangent_epb) {
     case 2: launch_tangent_epb<2>(c, precision); break;
     case 4: launch_tangent_epb<4>(c, precision); break;

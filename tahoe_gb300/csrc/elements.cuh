@@ -146,6 +146,17 @@ __device__ __forceinline__ void simo_roots(float d, float& J, float& invJ, float
   sc = powf(J, -2.0f / 3.0f);
 }
 
+// the isotropic modulus matrix of E and nu (or of equal entries)
+inline bool isotropic_moduli(const MatParams& m) {
+  const double l = m.C[1], g = m.C[21];
+  for (int i = 0; i < 6; ++i)
+    for (int j = 0; j < 6; ++j) {
+      const double want = i < 3 && j < 3 ? (i == j ? l + 2.0 * g : l) : (i == j ? g : 0.0);
+      if (m.C[i * 6 + j] != want) return false;
+    }
+  return true;
+}
+
 struct J2View {
   int8_t* flags;
   int8_t* alloc;

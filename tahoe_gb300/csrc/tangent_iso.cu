@@ -295,17 +295,6 @@ __global__ void __launch_bounds__(kIsoThreads, 3)
   iso_rows<FS, HAVEN>(rec + lane, Ke, tid >> 5, e, live);
 }
 
-// the isotropic modulus matrix of E and nu (or of equal entries)
-bool isotropic(const MatParams& m) {
-  const double l = m.C[1], g = m.C[21];
-  for (int i = 0; i < 6; ++i)
-    for (int j = 0; j < 6; ++j) {
-      const double want = i < 3 && j < 3 ? (i == j ? l + 2.0 * g : l) : (i == j ? g : 0.0);
-      if (m.C[i * 6 + j] != want) return false;
-    }
-  return true;
-}
-
 template <bool FS, bool HAVEN>
 int launch_t(Context* c, float* Ke, const J2View& j2) {
   const size_t dyn = sizeof(float) * (8 * kRec * kIsoElems + 2 * 8 * 3 * (kIsoElems + 1));
@@ -336,7 +325,8 @@ int launch_form(Context* c, float* Ke) {
 
 // Total-Lagrangian Simo groups and small-strain groups of isotropic Hookean
 // and J2 blocks without B-bar.  The others (B-bar's mean gradients, the updated
-// configuration, anisotropic and St.Venant moduli) keep the general kernel.
+// configuration, anisotropic moduli) keep the general kernel; St.Venant groups
+// and FP64: tangent_blocks.cu.
 bool tangent_iso_applies(const Context* c, int precision) {
   if (precision != TG_MIXED || c->nel <= 0) return false;
   const int nb = c->have_blocks ? c->mats.nblocks : 1;
@@ -345,7 +335,7 @@ bool tangent_iso_applies(const Context* c, int precision) {
   for (int b = 0; b < nb; ++b) {
     const MatParams& m = c->mats.m[b];
     if (fs ? m.kind != TG_MAT_FS_SIMO
-           : !((m.kind == TG_MAT_SS_HOOKEAN || m.kind == TG_MAT_SS_J2) && isotropic(m)))
+           : !((m.kind == TG_MAT_SS_HOOKEAN || m.kind == TG_MAT_SS_J2) && isotropic_moduli(m)))
       return false;
   }
   return true;

@@ -467,6 +467,9 @@ int launch_tangent(Context* c, int precision);   // Ke per element
 // the same for moduli of the isotropic form (tangent_iso.cu)
 bool tangent_iso_applies(const Context* c, int precision);
 int launch_tangent_iso(Context* c);
+// the same in FP64, and St.Venant groups in both (tangent_blocks.cu)
+bool tangent_blocks_applies(const Context* c, int precision);
+int launch_tangent_blocks(Context* c, int precision);
 int launch_assemble(Context* c, int precision);
 int launch_blob_structure(Context* c, int precision);
 // segmented (per-RVE) reductions over node / element ranges
