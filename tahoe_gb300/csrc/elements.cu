@@ -1059,8 +1059,7 @@ void launch_tangent_epb(Context* c, int precision) {
 
 int launch_tangent(Context* c, int precision) {
   if (tangent_iso_applies(c, precision)) return launch_tangent_iso(c);
-  // another number of elements per CTA asks for the general kernel
-  if (c->tangent_epb == kTanElems && tangent_blocks_applies(c, precision)) return launch_tangent_blocks(c, precision);
+  if (tangent_blocks_applies(c, precision)) return launch_tangent_blocks(c, precision);
   switch (c->tangent_epb) {
     case 2: launch_tangent_epb<2>(c, precision); break;
     case 4: launch_tangent_epb<4>(c, precision); break;

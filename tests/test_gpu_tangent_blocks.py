@@ -21,10 +21,17 @@ MATS = {
 }
 
 
-@pytest.mark.parametrize("nel", [1, 7, 8, 9, 33])
-@pytest.mark.parametrize("kind,precision", [("simo", lib.FP64), ("stvenant", lib.FP64), ("stvenant", lib.MIXED),
-                                            ("j2", lib.FP64), ("hooke", lib.FP64)])
-def test_equals_the_general_kernel(nel, kind, precision):
+# an unused block of a material that the kernel does not take sends a group to
+# the general one
+OTHER = {
+    "simo": {"kind": "fs_stvenant", "E": 1.0, "nu": 0.2},
+    "stvenant": {"kind": "fs_simo", "mu": 1.0, "kappa": 1.0},
+    "j2": {"kind": "ss_hookean", "C": np.diag([3.0, 4.0, 5.0, 1.0, 1.5, 2.0]).reshape(36)},
+}
+OTHER["hooke"] = OTHER["j2"]
+
+
+def _context(nel, kind, general):
     formulation, mats, amplitude = MATS[kind]
     mesh = BoxMesh(nel, 1, 1, lx=nel, jitter=0.0)
     rng = np.random.default_rng(nel)
@@ -32,25 +39,36 @@ def test_equals_the_general_kernel(nel, kind, precision):
     c = lib.Context(0)
     c.upload(X, mesh.conn, equations(len(X), []))
     c.set_formulation(formulation)
-    for b, m in enumerate(mats):
+    for b, m in enumerate(mats + [OTHER[kind]] * general):
         c.set_material(b, *material_params(m))
     c.set_blocks(np.arange(nel) % len(mats))
     c.set_u(rng.uniform(-amplitude, amplitude, size=X.shape))
     c.set_iteration(0)
     c.residual(want_vector=False)  # J2: the yielding points of this state
+    return c, X
+
+
+@pytest.mark.parametrize("nel", [1, 7, 8, 9, 33])
+@pytest.mark.parametrize("kind,precision", [("simo", lib.FP64), ("stvenant", lib.FP64), ("stvenant", lib.MIXED),
+                                            ("j2", lib.FP64), ("hooke", lib.FP64)])
+def test_equals_the_general_kernel(nel, kind, precision):
+    c, X = _context(nel, kind, 0)
     c.tangent(precision)
     v = c.tangent_csr()[2]
-    c.tangent_config(4)  # the general kernel
-    c.tangent(lib.FP64)
-    ref = c.tangent_csr()[2]
+    g, _ = _context(nel, kind, 1)
+    g.tangent(lib.FP64)
+    ref = g.tangent_csr()[2]
     # sums of 8 points of products of at most 20 factors of order one: 200
     # roundings of 2^-53 (2^-24) of the largest entry
     eps = 2.0**-53 if precision == lib.FP64 else 2.0**-24
     assert np.abs(v - ref).max() <= 200 * eps * np.abs(ref).max()
-    u = np.zeros(X.shape)
-    u[:, 0] = -2.0 * X[:, 0]
-    if formulation == lib.TOTAL_LAGRANGIAN:  # turned inside out
-        c.tangent_config(8)
+    for epb in (2, 4):  # bitwise the same for every launch shape
+        c.tangent_config(epb)
+        c.tangent(precision)
+        assert np.array_equal(c.tangent_csr()[2], v)
+    if MATS[kind][0] == lib.TOTAL_LAGRANGIAN:  # turned inside out
+        u = np.zeros(X.shape)
+        u[:, 0] = -2.0 * X[:, 0]
         c.set_u(u)
         with pytest.raises(lib.TahoeError):
             c.tangent(precision)
