@@ -78,6 +78,7 @@ __global__ void segment_combine_kernel(int nseg, const int* __restrict__ off, co
 
 constexpr int kNormShare = 2048;   // nodes
 constexpr int kStressShare = 256;  // elements
+constexpr int kMacroShare = 64;    // elements
 
 __global__ void __launch_bounds__(256) segment_norms_kernel(int nseg, const int* __restrict__ off,
                                                             const double4_32a* __restrict__ R,
@@ -146,20 +147,23 @@ __device__ __forceinline__ int upper_slot_of(int a, int b) { return a * 8 - a * 
 
 // Column kL of every RVE's macro tangent: sum over the RVE's element nodes of
 // (K_e w_e)_a (x) X_a, from the staged element matrices (36 upper node-pair
-// blocks; lower blocks by symmetry).  Written to out[seg*81 + jJ*9 + kL].
+// blocks; lower blocks by symmetry).  Partials of a share of kMacroShare
+// elements: a CTA per RVE and column left the chip waiting for the largest
+// RVEs (48 RVEs of sides 4 to 12 in FP64: 1.50 ms, in shares 0.69).
 template <typename T>
 __global__ void __launch_bounds__(256) segment_macro_kernel(int nseg, const int* __restrict__ eoff,
                                                             const int* __restrict__ conn, const double* __restrict__ X,
                                                             int nnd, const T* __restrict__ Ke,
-                                                            const double4_32a* __restrict__ w_all, int kL0,
-                                                            const double* __restrict__ vol0, double* __restrict__ out) {
-  // grid rows (blockIdx.y) are the columns kL0 + y, each with its own w
-  const int kL = kL0 + blockIdx.y;
+                                                            const double4_32a* __restrict__ w_all,
+                                                            double* __restrict__ part) {
+  // grid rows (blockIdx.y) are the columns, each with its own w
   const double4_32a* __restrict__ w = w_all + (long long)blockIdx.y * nnd;
-  for (int sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
+  int sg, e0, e1;
+  if (!share_of<kMacroShare>(blockIdx.x, nseg, eoff, sg, e0, e1)) return;
+  {
     double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    const long long k0 = (long long)eoff[sg] * 8, k1 = (long long)eoff[sg + 1] * 8;
-    for (long long k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+    const long long k1 = (long long)e1 * 8;
+    for (long long k = (long long)e0 * 8 + threadIdx.x; k < k1; k += blockDim.x) {
       const long long e = k >> 3;
       const int a = (int)(k & 7);
       const int* ce = conn + e * 8;
@@ -190,12 +194,23 @@ __global__ void __launch_bounds__(256) segment_macro_kernel(int nseg, const int*
       }
     }
     cta_sum<9>(v);
-    if (threadIdx.x == 0) {
-      const double s = vol0 ? 1.0 / vol0[sg] : 1.0;
+    if (threadIdx.x == 0)
 #pragma unroll
-      for (int jJ = 0; jJ < 9; ++jJ) out[(long long)sg * 81 + jJ * 9 + kL] = v[jJ] * s;
-    }
+      for (int jJ = 0; jJ < 9; ++jJ) part[((long long)blockIdx.x * gridDim.y + blockIdx.y) * 9 + jJ] = v[jJ];
   }
+}
+
+// out[sg*81 + jJ*9 + kL0 + column]: the sum of the shares' partials in order
+__global__ void segment_macro_combine_kernel(int nseg, const int* __restrict__ off, int ncols,
+                                             const double* __restrict__ part, int kL0,
+                                             const double* __restrict__ vol0, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nseg * ncols * 9) return;
+  const int sg = i / (ncols * 9), v = i % (ncols * 9), col = v / 9, jJ = v % 9;
+  const int b0 = off[sg] / kMacroShare + sg, n = (off[sg + 1] - off[sg] + kMacroShare - 1) / kMacroShare;
+  double a = 0.0;
+  for (int b = 0; b < n; ++b) a += part[(long long)(b0 + b) * (ncols * 9) + v];
+  out[(long long)sg * 81 + jJ * 9 + kL0 + col] = a * (vol0 ? 1.0 / vol0[sg] : 1.0);
 }
 
 }  // namespace
@@ -219,15 +234,22 @@ int launch_macro_combine(Context* c, const double4_32a* d_v, double4_32a* d_w) {
 
 int launch_segment_macro(Context* c, const double4_32a* d_w, int kL, int ncols, const double* d_vol0,
                          double* d_out) {
-  const dim3 grid(std::min(c->nseg, c->num_sms * 16), ncols);
+  const int nb = share_blocks(c->nel, c->nseg, kMacroShare);
+  const dim3 grid(nb, ncols);
+  double* part = nullptr;
+  if (!ok(c, cudaMallocAsync((void**)&part, sizeof(double) * 9 * nb * ncols, c->stream), "alloc")) return TG_ERR_OOM;
   if (c->tangent_precision == TG_MIXED)
     segment_macro_kernel<float><<<grid, 256, 0, c->stream>>>(c->nseg, c->d_seg_elem, c->d_conn, c->d_X, c->nnd,
-                                                             c->d_Ke32, d_w, kL, d_vol0, d_out);
+                                                             c->d_Ke32, d_w, part);
   else
     segment_macro_kernel<double><<<grid, 256, 0, c->stream>>>(c->nseg, c->d_seg_elem, c->d_conn, c->d_X, c->nnd,
-                                                              c->d_Ke64, d_w, kL, d_vol0, d_out);
-  c->launches++;
-  return ok(c, cudaGetLastError(), "segment_macro_kernel") ? TG_OK : TG_ERR_CUDA;
+                                                              c->d_Ke64, d_w, part);
+  segment_macro_combine_kernel<<<(c->nseg * ncols * 9 + 127) / 128, 128, 0, c->stream>>>(c->nseg, c->d_seg_elem, ncols,
+                                                                                        part, kL, d_vol0, d_out);
+  c->launches += 2;
+  const int s = ok(c, cudaGetLastError(), "segment_macro_kernel") ? TG_OK : TG_ERR_CUDA;
+  cudaFreeAsync(part, c->stream);
+  return s;
 }
 
 int launch_segment_norms(Context* c, int nseg, const int* d_node_off, double* d_out) {
