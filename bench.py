@@ -447,6 +447,8 @@ def run_ours(args):
                       "assembly": round(t_asm, 4), "residual": round(t_res, 4),
                       "residual_fp64": round(t_res64, 4)},
         "roofline": {"kernel": product,
+                     "note": "the streamed product of the form; the default solve of this mesh is one launch of "
+                             "hybrid_kernel, which reads 217 MB an iteration (profiles/hybrid_pcg_c2_64cubed.md)",
                      "storage": "symmetric push" if push else "symmetric" if sym else "full", "bound": "hbm", "achieved": round(achieved, 1),
                      "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4), "peak_kind": peak_kind,
                      "algorithmic_bytes": int(bytes_spmv),

@@ -181,9 +181,9 @@ int tg_apply_update(tg_context* ctx);
  * driver context).  All calls on a device share the array: calls that overlap
  * on the GPU race.  The solve reads the full matrix storage: a tangent formed
  * for the push storage alone (tg_pcg_form 3; the default picks it only on
- * meshes of a million block nonzeros and more, above this call's limit) has
- * its full storage assembled, and allocated if it never was, by the first
- * call. */
+ * meshes of a million block nonzeros and more, above this call's limit) or
+ * not at all (the default form solves such meshes without a storage) has its
+ * full storage assembled, and allocated if it never was, by the first call. */
 int tg_pcg_solve_noalloc(tg_context* ctx, const double* rhs_device, double* du_device, double rel_tol, int max_it,
                          int precond, int* iterations, double* rel_res);
 
@@ -313,8 +313,10 @@ int tg_segment_solver(tg_context* ctx, int per_rve);
  * K_ii du_i = -K_ib (dF X)_b is solved (PCG with params' precision,
  * preconditioner, lin_rel_tol, lin_max_it) and dP = (1/V0) sum_a (K du)_a (x)
  * X_a.  C is nseg*81 doubles, C[s*81 + (3j+J)*9 + (3k+L)] = dP_jJ/dF_kL;
- * vol0 as for tg_segment_average_stress.  The nine solves run as one
- * multi-vector PCG over the whole batch: each right-hand side stops when its
+ * vol0 as for tg_segment_average_stress.  RVEs that the default
+ * form solves on the chip (tg_pcg_form) take nine such solves each, every one
+ * to lin_rel_tol of its own right-hand side.  Otherwise the nine solves run as
+ * one multi-vector PCG over the whole batch: each right-hand side stops when its
  * residual norm over the batch falls below lin_rel_tol times its initial
  * norm over the batch (not per RVE), so an RVE's tangent in a batch agrees
  * with the same RVE's tangent computed alone to about lin_rel_tol times the
@@ -410,13 +412,18 @@ int tg_spmv_release(tg_context* ctx, int per_warp);
  * product in a slot of its lower row, which the vector kernel adds in a fixed
  * order (bitwise repeatable; it differs from form 1 by rounding).  The
  * storage is built on the device on first use after a mesh change and its
- * values are copied from every new assembly.  form = -1 (default): form 3
- * on meshes of at least one million block nonzeros, form 1 below (where the
- * one-time build of the push storage is not amortised).  The symmetric
- * format of tg_spmv_symmetric, segmented batches and the no-allocation entry
- * point use their own kernels. */
+ * values are copied from every new assembly.  form = -1 (default): one launch
+ * per solve, the rows assembled from the element blocks and kept on the chip,
+ * for RVEs and meshes that fit it (in FP64 up to about 25,000 nodes), and in
+ * mixed precision up to about 340,000 nodes with the rest of the matrix read
+ * from L2 and device memory; the same recurrences as form 1, bitwise
+ * repeatable, different from it by rounding.  Above, and where device memory
+ * for it is short: form 3 on meshes of at least one million block nonzeros,
+ * form 1 below.  The symmetric format of tg_spmv_symmetric and the
+ * no-allocation entry point use their own kernels. */
 int tg_pcg_form(tg_context* ctx, int form);
-/* the form the next single-vector solve runs on the current mesh (0..3) */
+/* the streamed form of the next single-vector solve on the current mesh
+ * (0..3); with form -1 the one it takes where it does not solve on the chip */
 int tg_pcg_form_get(const tg_context* ctx, int* form);
 /* L2 priorities of the streamed matrix.  bytes >= 0: the leading whole
  * tiles within `bytes` of the matrix storage are copied with evict_last
@@ -437,7 +444,7 @@ int tg_spmv_l2_keep(tg_context* ctx, long long bytes);
  * default 512).  The results equal the full-storage product up to the order
  * of the FP sums. */
 int tg_spmv_symmetric(tg_context* ctx, int on, int tile_blocks);
-/* elements per CTA of the tangent kernel: 2, 4 or 8 (default 8); element
+/* elements per CTA of the general tangent kernel: 2, 4 or 8 (default 8); element
  * matrices are bitwise the same for every choice */
 int tg_tangent_config(tg_context* ctx, int elems_per_block);
 /* the current launch shapes (any pointer may be NULL) */

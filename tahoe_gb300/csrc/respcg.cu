@@ -1,11 +1,12 @@
 // Resident PCG, sm_103a: a whole (block-)Jacobi CG solve in one launch with
-// the matrix held in shared memory.
+// the matrix held on the SMs.
 //
-// A matrix that fits the chip's shared memory is read once per solve instead
-// of once per iteration: every CTA assembles the rows of its part straight
-// from the element blocks into shared memory and keeps them there, its rows'
-// vectors live in registers, and the iterations touch nothing but shared
-// memory and the words the CTAs exchange.  Two forms, one kernel body:
+// A matrix that fits the chip's registers, tensor memory and shared memory is
+// read once per solve instead of once per iteration: every CTA assembles the
+// rows of its part straight from the element blocks and keeps them there, and
+// the iterations touch nothing but them and the words the CTAs exchange
+// (ResShape, respcg_device.cuh, says which chunk lies where).  Two forms, one
+// kernel body:
 //
 //   cluster  k <= 16 CTAs of one thread-block cluster per solve; the new
 //            search vector and the partial sums go to the other CTAs as
@@ -29,11 +30,14 @@
 // alone: a solve is bitwise repeatable and an RVE's does not depend on the
 // batch it shares.
 //
-// Measured against the streamed kernels (product + vector kernel, 14 us an
-// iteration on a 37x29x23 block, 20 us on a 16^3 FP64 cube; four kernels and
-// 26 us on one RVE of side 8): 7.5, 10.5 and 5 us, with no host round trip
-// inside a solve.  What bounds an iteration: the shared-memory reads of the
-// values (FP32) or the FP64 pipe, then the latency of the two exchanges.
+// Measured against the streamed kernels (product + vector kernel: 20 us an
+// iteration on a 16^3 FP64 cube, 39 on a 28^3 one; four kernels and 26 us on
+// one RVE of side 8): 9.4, 24.2 and 4.6 us, with no host round trip inside a
+// solve; 4,096 RVEs 540 -> 221 ms with stress, tangent and residuals.  What
+// bounds an iteration: of 12,300 cycles of an RVE of side 15 in a cluster 4,900
+// are the product (shared-memory reads), 1,200 the update and the rest the
+// latency of the exchanges and sums; in FP64 the FP64 pipe.  Whole FP32 meshes
+// of 20,000 nodes and more: hybridpcg.cu.
 //
 // Rows and storage: a warp holds chunks of 8 consecutive active rows, 4 lanes per row;
 // lane l takes blocks l, l+4, ... of its row (sliced ELL per warp: step t of

@@ -175,8 +175,9 @@ class Context:
         self.sym_mode = 0
 
     def product_kernel(self):
-        """Name of the kernel the single-vector solve multiplies with (a
-        segmented batch: the kernel of its per-RVE solves)."""
+        """Name of the streamed product kernel of the single-vector solve's
+        form (a segmented batch: of its per-RVE solves); the default form
+        streams only what it does not solve on the chip."""
         segmented = getattr(self, "nseg", 0) > 0
         form = self.effective_form()
         if segmented:
@@ -508,13 +509,15 @@ class Context:
         """Recurrences of the single-vector PCG: 3 single-reduction with
         programmatic launch dependencies on the symmetric push storage, 1 the
         same on the full storage, 2 form 1 without programmatic dependencies,
-        0 textbook, -1 (default) form 3 on meshes of at least a million block
-        nonzeros and form 1 below."""
+        0 textbook, -1 (default) one launch per solve with the matrix on the
+        chip where it fits (tahoe_gb300.h), else form 3 on meshes of at least
+        a million block nonzeros and form 1 below."""
         self._chk(self.L.tg_pcg_form(self.h, int(form)), "tg_pcg_form")
         self.form = int(form)
 
     def effective_form(self):
-        """The form the next single-vector solve runs on the current mesh."""
+        """The streamed form of the next single-vector solve on the current
+        mesh (default form: where it does not solve on the chip)."""
         f = ctypes.c_int(0)
         self._chk(self.L.tg_pcg_form_get(self.h, ctypes.byref(f)), "tg_pcg_form_get")
         return f.value
