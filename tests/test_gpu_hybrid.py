@@ -67,3 +67,27 @@ def test_hybrid_solve_equals_the_streamed_solve(dims):
         _, cut, _, rc2 = c.pcg(R, rel_tol=tol, max_it=7, precond=precond)
         assert cut == 7 and rc2 != 0
 
+
+
+def test_contexts_on_two_threads():
+    # two cooperative launches at a time, each of every SM
+    import threading
+
+    systems = [_system((37, 29, 23)), _system((50, 48, 30))]
+    alone = [c.pcg(R, rel_tol=1e-6, max_it=5000) for _, c, R in systems]
+    got = [[], []]
+
+    def work(i):
+        _, c, R = systems[i]
+        for _ in range(6):
+            got[i].append(c.pcg(R, rel_tol=1e-6, max_it=5000))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(2):
+        assert len(got[i]) == 6
+        for du, its, _, rc in got[i]:
+            assert rc == 0 and its == alone[i][1] and np.array_equal(du, alone[i][0])
