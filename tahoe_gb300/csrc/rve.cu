@@ -149,7 +149,7 @@ __device__ __forceinline__ int upper_slot_of(int a, int b) { return a * 8 - a * 
 // (K_e w_e)_a (x) X_a, from the staged element matrices (36 upper node-pair
 // blocks; lower blocks by symmetry).  Partials of a share of kMacroShare
 // elements: a CTA per RVE and column left the chip waiting for the largest
-// RVEs (48 RVEs of sides 4 to 12 in FP64: 1.50 ms, in shares 0.69).
+// RVEs (48 RVEs of sides 4 to 12 in FP64: 1.50 ms, in shares 0.52).
 template <typename T>
 __global__ void __launch_bounds__(256) segment_macro_kernel(int nseg, const int* __restrict__ eoff,
                                                             const int* __restrict__ conn, const double* __restrict__ X,
@@ -172,17 +172,15 @@ __global__ void __launch_bounds__(256) segment_macro_kernel(int nseg, const int*
 #pragma unroll
       for (int b = 0; b < 8; ++b) {
         const double4_32a wb = w[ce[b]];
-        if (a <= b) {
-          const T* B = Kb + upper_slot_of(a, b) * kKeBlock;
-          y0 += (double)B[0] * wb.x + (double)B[1] * wb.y + (double)B[2] * wb.z;
-          y1 += (double)B[4] * wb.x + (double)B[5] * wb.y + (double)B[6] * wb.z;
-          y2 += (double)B[8] * wb.x + (double)B[9] * wb.y + (double)B[10] * wb.z;
-        } else {
-          const T* B = Kb + upper_slot_of(b, a) * kKeBlock;
-          y0 += (double)B[0] * wb.x + (double)B[4] * wb.y + (double)B[8] * wb.z;
-          y1 += (double)B[1] * wb.x + (double)B[5] * wb.y + (double)B[9] * wb.z;
-          y2 += (double)B[2] * wb.x + (double)B[6] * wb.y + (double)B[10] * wb.z;
-        }
+        // the block or its transpose, chosen before the arithmetic: a warp
+        // pays the FP64 pipe for either branch
+        const bool up = a <= b;
+        const T* B = Kb + (up ? upper_slot_of(a, b) : upper_slot_of(b, a)) * kKeBlock;
+        const T m00 = B[0], m11 = B[5], m22 = B[10], m01 = B[up ? 1 : 4], m02 = B[up ? 2 : 8], m10 = B[up ? 4 : 1],
+                m12 = B[up ? 6 : 9], m20 = B[up ? 8 : 2], m21 = B[up ? 9 : 6];
+        y0 += (double)m00 * wb.x + (double)m01 * wb.y + (double)m02 * wb.z;
+        y1 += (double)m10 * wb.x + (double)m11 * wb.y + (double)m12 * wb.z;
+        y2 += (double)m20 * wb.x + (double)m21 * wb.y + (double)m22 * wb.z;
       }
       const int n = ce[a];
       const double Xn[3] = {X[n], X[nnd + n], X[2 * nnd + n]};
