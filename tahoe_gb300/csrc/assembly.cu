@@ -308,6 +308,10 @@ int ensure_full_assembly(Context* c) {
   if (precision != TG_MIXED && precision != TG_FP64) return TG_OK;
   long long& serial = precision == TG_MIXED ? c->full_serial32 : c->full_serial64;
   if (serial == c->tangent_serial) return TG_OK;
+  if ((precision == TG_MIXED ? c->ke_serial32 : c->ke_serial64) < 0) {
+    c->err = "the element blocks of the last tangent were overwritten: form a tangent first";
+    return TG_ERR_ARG;
+  }
   int s = ensure_blob(c, precision);
   if (!s) s = launch_assemble(c, precision);
   if (!s) serial = c->tangent_serial;

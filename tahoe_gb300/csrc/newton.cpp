@@ -110,13 +110,19 @@ int form_tangent(Context* c, int precision) {
     if (!c->d_Ke64 && !dalloc(c, &c->d_Ke64, keN)) return TG_ERR_OOM;
     if (!c->d_minv64 && !dalloc(c, &c->d_minv64, minv_values(c->nnd))) return TG_ERR_OOM;
   }
-  int s = launch_tangent(c, precision);
+  // every buffer before the element blocks are overwritten: a tangent that
+  // finds no room leaves the last one as it was
   bool resident = false;
-  if (!s) s = resident_active(c, precision, &resident);
+  int s = resident_active(c, precision, &resident);
+  const bool push = !resident && push_solve(c);
+  if (!s && !resident) s = push ? push_structure(c, precision) : ensure_blob(c, precision);
+  if (s) return s;
+  (precision == TG_MIXED ? c->ke_serial32 : c->ke_serial64) = -1;
+  s = launch_tangent(c, precision);
   if (!s && resident) {
     // the solve assembles its rows from the element blocks itself
     ++c->tangent_serial;
-  } else if (!s && push_solve(c)) {
+  } else if (!s && push) {
     // the solve streams the push storage: its upper blocks are assembled
     // straight into it, the full storage only when something reads it
     s = launch_assemble_upper(c, precision);
@@ -125,8 +131,7 @@ int form_tangent(Context* c, int precision) {
       (precision == TG_MIXED ? c->push.serial32 : c->push.serial64) = c->tangent_serial;
     }
   } else if (!s) {
-    s = ensure_blob(c, precision);
-    if (!s) s = launch_assemble(c, precision);
+    s = launch_assemble(c, precision);
     if (!s) {
       ++c->tangent_serial;
       (precision == TG_MIXED ? c->full_serial32 : c->full_serial64) = c->tangent_serial;

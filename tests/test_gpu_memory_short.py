@@ -1,0 +1,59 @@
+"""Short device memory: a tangent that finds no room leaves the last one as it
+was."""
+import numpy as np
+import pytest
+
+from tahoe_gb300 import lib
+from tahoe_gb300.meshgen import BoxMesh, equations
+from tahoe_gb300.model import material_params
+from tests.memory import ShortMemory
+
+pytestmark = pytest.mark.gpu
+
+SIMO = {"kind": "fs_simo", "mu": 1.0, "kappa": 10.0}
+
+
+def _context(n=16):
+    mesh = BoxMesh(n, n, n, jitter=0.1, seed=2)
+    bottom = mesh.face_nodes(2, 0)
+    eq = equations(mesh.nnd, np.concatenate([bottom * 3 + d for d in range(3)]))
+    c = lib.Context(0)
+    c.upload(mesh.X, mesh.conn, eq)
+    c.set_formulation(lib.TOTAL_LAGRANGIAN)
+    c.set_material(0, *material_params(SIMO))
+    f = np.zeros((mesh.nnd, 3))
+    f[mesh.face_nodes(2, 1), 0] = 1e-4
+    c.set_fext(f)
+    c.set_load_factor(1.0)
+    c.set_u(np.zeros((mesh.nnd, 3)))
+    c.residual(want_vector=False)
+    return c, mesh
+
+
+def _solve(c):
+    return c.pcg(None, rel_tol=1e-6, max_it=2000)[0]
+
+
+@pytest.mark.parametrize("precision", [lib.FP64, lib.MIXED])
+@pytest.mark.parametrize("form", [1, 3])
+def test_tangent_without_room_leaves_the_last_one(precision, form):
+    """The default form solves this mesh without a matrix storage; the streamed
+    form's storage then finds no room, at another displacement."""
+    c, mesh = _context()
+    c.tangent(precision)
+    ref = _solve(c)
+    c.set_u(0.02 * mesh.X * np.array([1.0, -0.3, 0.2]))
+    c.pcg_form(form)
+    with ShortMemory():
+        with pytest.raises(lib.TahoeError) as e:
+            c.tangent(precision)
+        assert e.value.code == -3
+    c.pcg_form(-1)
+    assert np.array_equal(_solve(c), ref)
+    # streamed: the same matrix, assembled from the same element blocks
+    c.pcg_form(form)
+    du = _solve(c)
+    assert np.abs(du - ref).max() < 1e-3 * np.abs(ref).max()
+    # and the tangent that found no room is the next one's
+    c.tangent(precision)
+    assert np.abs(_solve(c) - ref).max() > 1e-3 * np.abs(ref).max()
