@@ -996,13 +996,38 @@ int resident_slots(Context* c, long long n, const int* d_blk, const int* d_cptr,
 }
 
 namespace {
+// A device buffer of a mode's plans.
+template <typename T>
+bool hold(Context* c, ResMode& M, T** p, size_t n) {
+  if (!dalloc(c, p, n)) return false;
+  M.bufs.push_back((void*)*p);
+  return true;
+}
+void drop_mode(Context* c, ResMode& M) {
+  for (void* p : M.bufs) dfree(c, p);
+  M = ResMode{};
+}
+
 // Rows of the whole mesh on the device; R receives what the split needs.
-int rows_of_mesh(Context* c, ResRows& R, ResPlanDev& D) {
+int rows_of_mesh(Context* c, ResMode& M, ResRows& R, ResPlanDev& D) {
   R = ResRows{};
   const int n = c->nnd;
   cudaStream_t st = c->stream;
+  struct Scratch {
+    Context* c;
+    std::vector<void*> p;
+    ~Scratch() {
+      for (void* q : p) dfree(c, q);
+    }
+    bool get(int** q, size_t m) {
+      if (!dalloc(c, q, m)) return false;
+      p.push_back(*q);
+      return true;
+    }
+  } scratch{c, {}};
   int *flag = nullptr, *rank = nullptr, *tmp = nullptr, *node = nullptr;
-  if (!dalloc(c, &flag, (size_t)n) || !dalloc(c, &rank, (size_t)n + 1) || !dalloc(c, &tmp, (size_t)n / 1024 + 4))
+  if (!scratch.get(&flag, (size_t)n) || !scratch.get(&rank, (size_t)n + 1) ||
+      !scratch.get(&tmp, (size_t)n / 1024 + 4))
     return TG_ERR_OOM;
   rows_flag_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, c->d_mask, flag);
   int s = scan_counts(c, n, flag, rank, tmp);
@@ -1017,8 +1042,8 @@ int rows_of_mesh(Context* c, ResRows& R, ResPlanDev& D) {
   c->launches++;
   if (nch == 0) return TG_OK;
   int *cnt = nullptr, *step = nullptr, *lohi = nullptr;
-  if (!dalloc(c, &node, (size_t)R.rows) || !dalloc(c, &cnt, (size_t)nch) || !dalloc(c, &step, (size_t)nch + 1) ||
-      !dalloc(c, &lohi, 2 * (size_t)nch))
+  if (!hold(c, M, &node, (size_t)R.rows) || !scratch.get(&cnt, (size_t)nch) || !hold(c, M, &step, (size_t)nch + 1) ||
+      !scratch.get(&lohi, 2 * (size_t)nch))
     return TG_ERR_OOM;
   rows_node_kernel<<<(n + 255) / 256, 256, 0, st>>>(n, c->d_mask, rank, node);
   const int grid = (nch + 7) / 8;
@@ -1035,7 +1060,7 @@ int rows_of_mesh(Context* c, ResRows& R, ResPlanDev& D) {
   const size_t slots = (size_t)R.chunk_step[nch] * 32;
   int *blk = nullptr, *cidx = nullptr;
   int2* slot = nullptr;
-  if (!dalloc(c, &blk, slots) || !dalloc(c, &cidx, slots) || !dalloc(c, &slot, slots)) return TG_ERR_OOM;
+  if (!hold(c, M, &blk, slots) || !hold(c, M, &cidx, slots) || !hold(c, M, &slot, slots)) return TG_ERR_OOM;
   rows_chunk_kernel<true><<<grid, 256, 0, st>>>(R.rows, nch, node, c->d_rowptr, c->d_col, c->d_mask, rank, step, nullptr,
                                                 nullptr, blk, cidx);
   c->launches += 3;
@@ -1048,7 +1073,6 @@ int rows_of_mesh(Context* c, ResRows& R, ResPlanDev& D) {
   D.chunk_step = step;
   D.slot = slot;
   D.contrib = c->d_contrib;
-  for (int* p : {flag, rank, tmp, cnt, lohi}) dfree(c, p);
   return TG_OK;
 }
 }  // namespace
@@ -1081,20 +1105,14 @@ void resident_destroy(Context* c) {
 // A new partition into RVEs: the plans of the batch follow it.
 void resident_drop_batch(Context* c) {
   if (!c->res) return;
-  for (auto& a : c->res->mode) {
-    if (a[1].d_plans) dfree(c, a[1].d_plans);
-    a[1] = ResMode{};
-  }
+  for (auto& a : c->res->mode) drop_mode(c, a[1]);
 }
 
 namespace {
 
 // Plans the current mesh: every RVE of a batch (the template's plan for a
-// composed mesh) or the whole mesh.  A mesh that does not fit leaves the mode
-// at -1 and the streamed solves take it.
-int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
-  M = ResMode{};
-  M.state = -1;
+// composed mesh) or the whole mesh; M.state 1 where it fits.
+int plan_rows(Context* c, int precision, bool batch, ResMode& M) {
   const int elem = precision == TG_MIXED ? 4 : 8;
   ResLimits limits;
   int s = resident_limits(c, precision, &limits);
@@ -1124,13 +1142,13 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
     if ((long long)c->neq > 3LL * c->num_sms * chunks * kResChunkRows || c->neq == 0) return TG_OK;
     ResRows R;
     ResPlan P;
-    s = rows_of_mesh(c, R, P.dev);
+    s = rows_of_mesh(c, M, R, P.dev);
     if (s) return s;
     if (!resident_plan(R, elem, c->num_sms, limits, true, P)) return TG_OK;
     ResImage img;
     const size_t at = img.split_at(P);
     int* d = nullptr;
-    if (!dalloc(c, &d, img.data.size())) return TG_ERR_OOM;
+    if (!hold(c, M, &d, img.data.size())) return TG_ERR_OOM;
     if (!ok(c, cudaMemcpyAsync(d, img.data.data(), sizeof(int) * img.data.size(), cudaMemcpyHostToDevice, c->stream),
             "resident split") ||
         !ok(c, cudaStreamSynchronize(c->stream), "sync"))
@@ -1158,7 +1176,7 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
       M.plan_of.push_back(i);
     }
     int* d = nullptr;
-    if (!dalloc(c, &d, img.data.size())) return TG_ERR_OOM;
+    if (!hold(c, M, &d, img.data.size())) return TG_ERR_OOM;
     if (!ok(c, cudaMemcpyAsync(d, img.data.data(), sizeof(int) * img.data.size(), cudaMemcpyHostToDevice, c->stream),
             "resident rows") ||
         !ok(c, cudaStreamSynchronize(c->stream), "sync"))
@@ -1169,7 +1187,7 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
       resident_bind_split(D, d, at_split[i], M.plans[i]);
       D.contrib = c->d_contrib;
       int2* slot = nullptr;
-      if (!dalloc(c, &slot, std::max<size_t>(rows[i].blk.size(), 1))) return TG_ERR_OOM;
+      if (!hold(c, M, &slot, std::max<size_t>(rows[i].blk.size(), 1))) return TG_ERR_OOM;
       D.slot = slot;
       s = resident_slots(c, (long long)rows[i].blk.size(), D.blk, c->d_contrib_ptr, slot);
       if (s) return s;
@@ -1177,13 +1195,23 @@ int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
   }
   std::vector<ResPlanDev> dev;
   for (const ResPlan& P : M.plans) dev.push_back(P.dev);
-  if (!dalloc(c, &M.d_plans, std::max<size_t>(dev.size(), 1))) return TG_ERR_OOM;
+  if (!hold(c, M, &M.d_plans, std::max<size_t>(dev.size(), 1))) return TG_ERR_OOM;
   if (!ok(c, cudaMemcpyAsync(M.d_plans, dev.data(), sizeof(ResPlanDev) * dev.size(), cudaMemcpyHostToDevice, c->stream),
           "resident plans") ||
       !ok(c, cudaStreamSynchronize(c->stream), "sync"))
     return TG_ERR_CUDA;
   M.state = 1;
   return TG_OK;
+}
+// A mesh that does not fit the chip keeps nothing: mode -1, and the streamed
+// solves take it.
+int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
+  drop_mode(c, M);
+  const int s = plan_rows(c, precision, batch, M);
+  if (!s && M.state == 1) return TG_OK;
+  drop_mode(c, M);
+  M.state = -1;
+  return s;
 }
 
 int aux_streams(Context* c) {

@@ -72,6 +72,7 @@ struct ResMode {
   std::vector<ResPlan> plans;
   std::vector<int> plan_of;  // plan of every RVE (one entry for a whole mesh)
   ResPlanDev* d_plans = nullptr;
+  std::vector<void*> bufs;   // its device buffers
 };
 // Everything the resident PCG keeps with a context: device buffers go with the
 // mesh, streams and events with the context.
