@@ -94,6 +94,11 @@ bool talloc(Context* c, MeshTemplate* t, T** p, size_t n) {
   return true;
 }
 
+void tfree(Context* c, MeshTemplate* t, void* p) {
+  cudaFreeAsync(p, c->stream);
+  t->allocs.erase(std::find(t->allocs.begin(), t->allocs.end(), p));
+}
+
 void release(Context* c, MeshTemplate* t) {
   for (void* p : t->allocs) cudaFreeAsync(p, c->stream);
   t->allocs.clear();
@@ -249,6 +254,8 @@ int template_resident(Context* c, int tpl, int precision, ResPlan& P, bool& fits
   MeshTemplate* t = c->templates[tpl];
   const int p = precision == TG_MIXED ? 1 : 0;
   fits = false;
+  // no room for a plan: an error the caller streams on; the template is
+  // planned anew for its next batch
   auto put = [&](const ResImage& img, int** d) {
     if (!talloc(c, t, d, img.data.size())) return TG_ERR_OOM;
     return ok(c, cudaMemcpyAsync(*d, img.data.data(), sizeof(int) * img.data.size(), cudaMemcpyHostToDevice, c->stream),
@@ -267,7 +274,10 @@ int template_resident(Context* c, int tpl, int precision, ResPlan& P, bool& fits
     resident_bind_rows(t->res_dev, d, at, t->res_rows);
     t->res_dev.contrib = t->dev.contrib;
     int2* slot = nullptr;
-    if (!talloc(c, t, &slot, t->res_rows.blk.size())) return TG_ERR_OOM;
+    if (!talloc(c, t, &slot, t->res_rows.blk.size())) {
+      tfree(c, t, d);
+      return TG_ERR_OOM;
+    }
     t->res_dev.slot = slot;
     const int ss = resident_slots(c, (long long)t->res_rows.blk.size(), t->res_dev.blk, t->dev.cptr, slot);
     if (ss) return ss;

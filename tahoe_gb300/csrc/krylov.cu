@@ -1007,7 +1007,11 @@ int pcg_solve(Context* c, const double4_32a* d_rhs, double rel_tol, int max_it, 
     bool resident = false;
     const int sr = resident_active(c, c->tangent_precision, &resident);
     if (sr) return sr;
-    if (resident) return pcg_solve_resident(c, d_rhs, rel_tol, max_it, precond, iters, rel_res);
+    if (resident) {
+      const int s = pcg_solve_resident(c, d_rhs, rel_tol, max_it, precond, iters, rel_res);
+      if (s != TG_ERR_OOM) return s;
+      resident_refuse(c, c->tangent_precision);
+    }
   }
   // a solve that streams a matrix storage: its values (and the
   // preconditioner's) from the last tangent

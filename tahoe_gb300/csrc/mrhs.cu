@@ -645,7 +645,14 @@ int macro_tangent_mrhs(Context* c, int precision, int precond, double rel_tol, i
   if (!s && resident) {
     s = macro_solve_resident(c, precision, kNR, d_b, d_v, d_b, rel_tol, max_it, precond, iters);
     if (s == TG_ERR_NOT_CONVERGED) s = TG_OK;
-  } else if (!s) {
+    if (s == TG_ERR_OOM) {
+      resident_refuse(c, precision);
+      resident = false;
+      s = ensure_full_assembly(c);
+      if (!s) s = launch_lift_rhs(c, d_v, d_b, true, kNR);
+    }
+  }
+  if (!s && !resident) {
     s = precision == TG_MIXED ? mrhs_solve_t<float>(c, d_b, d_v, d_b, rel_tol, max_it, precond, iters, &worst)
                               : mrhs_solve_t<double>(c, d_b, d_v, d_b, rel_tol, max_it, precond, iters, &worst);
     if (s == TG_ERR_NOT_CONVERGED) s = TG_OK;

@@ -1203,15 +1203,15 @@ int plan_rows(Context* c, int precision, bool batch, ResMode& M) {
   M.state = 1;
   return TG_OK;
 }
-// A mesh that does not fit the chip keeps nothing: mode -1, and the streamed
-// solves take it.
+// A mesh that does not fit the chip, or whose plans find no room in device
+// memory, keeps nothing: mode -1, and the streamed solves take it.
 int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
   drop_mode(c, M);
   const int s = plan_rows(c, precision, batch, M);
   if (!s && M.state == 1) return TG_OK;
   drop_mode(c, M);
   M.state = -1;
-  return s;
+  return s == TG_ERR_OOM ? TG_OK : s;
 }
 
 int aux_streams(Context* c) {
@@ -1532,6 +1532,14 @@ int resident_active(Context* c, int precision, bool* on) {
   }
   *on = M.state > 0;
   return TG_OK;
+}
+
+// The mode of the next solve of a precision, given up: a solve found no room for
+// its buffers.
+void resident_refuse(Context* c, int precision) {
+  ResMode& M = c->res->mode[precision == TG_MIXED ? 1 : 0][c->nseg > 0 && c->seg_pcg_mode ? 1 : 0];
+  drop_mode(c, M);
+  M.state = -1;
 }
 
 int pcg_solve_resident(Context* c, const double4_32a* d_rhs, double rel_tol, int max_it, int precond, int* iters,

@@ -1,9 +1,9 @@
 """Short device memory: a tangent that finds no room leaves the last one as it
-was."""
+was, and what the solves on the chip find no room for is streamed."""
 import numpy as np
 import pytest
 
-from tahoe_gb300 import lib
+from tahoe_gb300 import lib, rve
 from tahoe_gb300.meshgen import BoxMesh, equations
 from tahoe_gb300.model import material_params
 from tests.memory import ShortMemory
@@ -57,3 +57,47 @@ def test_tangent_without_room_leaves_the_last_one(precision, form):
     # and the tangent that found no room is the next one's
     c.tangent(precision)
     assert np.abs(_solve(c) - ref).max() > 1e-3 * np.abs(ref).max()
+
+
+def _rves(composed):
+    ns, Fs = [16, 16], [rve.sample_F(np.random.default_rng(i)) for i in range(2)]
+    c = lib.Context(0)
+    if composed:
+        r = rve.ResidentRVEs(c)
+        r.compose(ns)
+        c.set_affine(np.asarray(Fs).reshape(-1))
+    else:
+        b = rve.RVEBatch(ns, Fs)
+        b.setup(ctx=c)
+        c.set_prescribed(b.prescribed_idx, b.prescribed_val)
+    c.residual(want_vector=False)
+    return c
+
+
+@pytest.mark.parametrize("precision", [lib.FP64, lib.MIXED])
+@pytest.mark.parametrize("case", ["mesh", "uploaded", "composed"])
+def test_plans_without_room_are_streamed(precision, case):
+    """A mesh whose matrix storage is there and whose plans for the solve on
+    the chip find no room: the streamed solve, bitwise."""
+    c = _context()[0] if case == "mesh" else _rves(case == "composed")
+    c.pcg_form(1 if case == "mesh" else 3)
+    if case != "mesh":
+        c.set_u(np.zeros((c.nnd, 3)))
+    c.tangent(precision)
+    ref = _solve(c)
+    c.pcg_form(-1)
+    with ShortMemory():
+        c.tangent(precision)
+        assert np.array_equal(_solve(c), ref)
+
+
+def test_exchange_without_room_is_streamed():
+    """The plans fit, the solve's exchange words do not."""
+    c, mesh = _context()
+    c.pcg_form(1)
+    c.tangent(lib.FP64)
+    ref = _solve(c)
+    c.pcg_form(-1)
+    c.tangent(lib.FP64)
+    with ShortMemory(left=200 << 10):
+        assert np.array_equal(_solve(c), ref)
