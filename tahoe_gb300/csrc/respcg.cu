@@ -1234,6 +1234,31 @@ int grow(Context* c, T** p, long long* cap, long long n) {
   return TG_OK;
 }
 
+// Launches of a batch's classes on streams beside the context's own.  The
+// context's stream waits for them on every way out: what it frees or
+// overwrites next is read by them.
+struct AuxStreams {
+  Context* c;
+  int n = 0;  // streams that follow the context's
+  int fork(int want) {
+    const int s = want > 0 ? aux_streams(c) : TG_OK;
+    if (s || want <= 0) return s;
+    if (!ok(c, cudaEventRecord(c->res->fork, c->stream), "fork")) return TG_ERR_CUDA;
+    for (; n < want; ++n)
+      if (!ok(c, cudaStreamWaitEvent(c->res->aux[n], c->res->fork, 0), "fork")) return TG_ERR_CUDA;
+    return TG_OK;
+  }
+  int join() {
+    bool good = true;
+    for (int a = 0; a < n; ++a)
+      good = ok(c, cudaEventRecord(c->res->join[a], c->res->aux[a]), "join") &&
+             ok(c, cudaStreamWaitEvent(c->stream, c->res->join[a], 0), "join") && good;
+    n = 0;
+    return good ? TG_OK : TG_ERR_CUDA;
+  }
+  ~AuxStreams() { join(); }
+};
+
 // Runs the solves of the listed RVEs (act; one for a whole mesh) for nvec
 // right-hand sides, nnd nodes apart in d_rhs and x, and reports each in out.
 // x is zero away from the solved rows.
@@ -1322,13 +1347,9 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
   // the classes run beside each other: each is small beside the chip's tail
   // otherwise
   const int naux = (int)std::min<size_t>(std::max<size_t>(cls.size(), 1) - 1, kResAux);
-  if (naux > 0) {
-    s = aux_streams(c);
-    if (s) return s;
-    if (!ok(c, cudaEventRecord(S.fork, st), "fork")) return TG_ERR_CUDA;
-    for (int q = 0; q < naux; ++q)
-      if (!ok(c, cudaStreamWaitEvent(S.aux[q], S.fork, 0), "fork")) return TG_ERR_CUDA;
-  }
+  AuxStreams beside{c};
+  s = beside.fork(naux);
+  if (s) return s;
   size_t first = 0;
   int q = 0;
   for (auto& e : cls) {
@@ -1367,9 +1388,8 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
       return TG_ERR_CUDA;
     ++q;
   }
-  for (int a = 0; a < naux; ++a)
-    if (!ok(c, cudaEventRecord(S.join[a], S.aux[a]), "join") || !ok(c, cudaStreamWaitEvent(st, S.join[a], 0), "join"))
-      return TG_ERR_CUDA;
+  s = beside.join();
+  if (s) return s;
   out.assign(std::max(n, 1), ResOut{});
   if (n && !ok(c, cudaMemcpyAsync(out.data(), S.d_out, sizeof(ResOut) * n, cudaMemcpyDeviceToHost, st), "out"))
     return TG_ERR_CUDA;
