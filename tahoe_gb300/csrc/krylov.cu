@@ -615,12 +615,7 @@ int ensure_vectors(Context* c, int precision) {
     *pp = v;
   }
   c->pcg_vec_precision = precision;
-  if (c->pcg_graph) {
-    cudaGraphExecDestroy(c->pcg_graph);
-    c->pcg_graph = nullptr;
-  }
-  c->pcg_graph_key = -1;
-  cg_free(c);  // its captured chunk names the old vectors
+  drop_graphs(c);  // every captured iteration names the old vectors
   return TG_OK;
 }
 
