@@ -608,8 +608,13 @@ template <typename T>
 int ensure_vectors(Context* c, int precision) {
   using V = typename Vec4<T>::type;
   if (c->pcg_vec_precision == precision) return TG_OK;
+  // of neither precision while they change: a failed allocation leaves some of
+  // either, and no update
+  c->pcg_vec_precision = -1;
+  c->have_du = false;
   for (void** pp : {&c->d_x, &c->d_r, &c->d_z, &c->d_p, &c->d_q}) {
     if (*pp) dfree(c, *pp);
+    *pp = nullptr;
     V* v = nullptr;
     if (!dalloc(c, &v, (size_t)c->nnd)) return TG_ERR_OOM;
     *pp = v;

@@ -420,7 +420,11 @@ int push_blob(Context* c, int precision) {
   // rank planes; slots no block pushes to (rows with fewer lower blocks
   // than the largest count) are never read
   unsigned char* pb = nullptr;
-  if (!dalloc(c, &pb, (size_t)std::max(ps.kmax, 1) * ps.pstride * vb)) return TG_ERR_OOM;
+  if (!dalloc(c, &pb, (size_t)std::max(ps.kmax, 1) * ps.pstride * vb)) {
+    dfree(c, *blob);  // both or neither: the blob says that both are there
+    *blob = nullptr;
+    return TG_ERR_OOM;
+  }
   *push = pb;
   if (!ok(c, cudaMemsetAsync(*blob, 0, (size_t)total, c->stream), "push blob")) return TG_ERR_CUDA;
   const int grid = std::max(1, std::min((c->nnd + 7) / 8, c->num_sms * 16));

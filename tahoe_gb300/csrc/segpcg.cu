@@ -473,6 +473,7 @@ int solve_seg_t(Context* c, const double4_32a* d_rhs, double rel_tol, int max_it
   if (s) return s;
   if (S.s_precision != precision || !S.d_s) {
     if (S.d_s) dfree(c, S.d_s);
+    S.d_s = nullptr;
     V* v = nullptr;
     if (!dalloc(c, &v, (size_t)c->nnd)) return TG_ERR_OOM;
     S.d_s = v;

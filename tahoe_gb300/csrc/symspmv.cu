@@ -451,10 +451,15 @@ int sym_convert(Context* c, int precision) {
   }
   const bool f32 = precision == TG_MIXED;
   const size_t pad = 16;  // V1 copies are rounded out to 16 bytes
-  if (f32 && !s.d_v8_32 && (!dalloc(c, &s.d_v8_32, (size_t)s.nu * 8) || !dalloc(c, &s.d_v1_32, (size_t)s.nu + pad)))
-    return TG_ERR_OOM;
-  if (!f32 && !s.d_v8_64 && (!dalloc(c, &s.d_v8_64, (size_t)s.nu * 8) || !dalloc(c, &s.d_v1_64, (size_t)s.nu + pad)))
-    return TG_ERR_OOM;
+  // both arrays of a precision or neither
+  auto values = [&](auto*& v8, auto*& v1) {
+    if (v8) return true;
+    if (dalloc(c, &v8, (size_t)s.nu * 8) && dalloc(c, &v1, (size_t)s.nu + pad)) return true;
+    if (v8) dfree(c, v8);
+    v8 = nullptr;
+    return false;
+  };
+  if (!(f32 ? values(s.d_v8_32, s.d_v1_32) : values(s.d_v8_64, s.d_v1_64))) return TG_ERR_OOM;
   const int grid = std::max(1, std::min((c->nnd + 7) / 8, c->num_sms * 16));
   if (f32)
     sym_convert_kernel<float><<<grid, 256, 0, c->stream>>>(

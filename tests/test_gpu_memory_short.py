@@ -101,3 +101,65 @@ def test_exchange_without_room_is_streamed():
     c.tangent(lib.FP64)
     with ShortMemory(left=200 << 10):
         assert np.array_equal(_solve(c), ref)
+
+
+def test_storages_are_whole_or_not_there():
+    """An allocation that fails between the arrays of one storage, at any of
+    them: the next use finds none or all of it."""
+    def ready(form):
+        c = _context()[0]
+        c.pcg_form(1)
+        c.tangent(lib.FP64)
+        ref = _solve(c)
+        c.pcg_form(form)
+        return c, ref
+
+    failed = 0
+    for left in range(1, 9):
+        # the push storage: tiles, then push slots
+        c, ref = ready(3)
+        with ShortMemory(left=left << 20):
+            try:
+                c.tangent(lib.FP64)
+            except lib.TahoeError as e:
+                assert e.code == -3
+                failed += 1
+        c.tangent(lib.FP64)
+        du = _solve(c)
+        assert np.abs(du - ref).max() < 1e-3 * np.abs(ref).max()
+        # the symmetric format: eight planes, then one
+        c, ref = ready(1)
+        with ShortMemory(left=left << 20):
+            try:
+                c.spmv_symmetric(1)
+            except lib.TahoeError as e:
+                assert e.code == -3
+                failed += 1
+        c.spmv_symmetric(1)
+        du = _solve(c)
+        assert np.abs(du - ref).max() < 1e-3 * np.abs(ref).max()
+    assert failed >= 8
+
+
+@pytest.mark.parametrize("left", [100, 200, 300, 400, 500, 600])
+def test_vectors_are_of_one_precision(left):
+    """An allocation that fails between the PCG vectors as they change their
+    precision: no update is left, and the next solve has all of them."""
+    c = _context()[0]
+    c.pcg_form(1)
+    c.tangent(lib.MIXED)
+    small = _solve(c)
+    c.tangent(lib.FP64)
+    ref = _solve(c)
+    c.tangent(lib.MIXED)
+    _solve(c)
+    c.tangent(lib.FP64)
+    with ShortMemory(left=left << 10):  # of five times 157 KB
+        with pytest.raises(lib.TahoeError) as e:
+            c.pcg(None, rel_tol=1e-6, max_it=2000, want_du=False)
+        assert e.value.code == -3
+        with pytest.raises(lib.TahoeError):
+            c.apply_update()
+    assert np.array_equal(_solve(c), ref)
+    c.tangent(lib.MIXED)
+    assert np.array_equal(_solve(c), small)
