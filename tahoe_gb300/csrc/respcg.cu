@@ -1167,6 +1167,7 @@ int plan_rows(Context* c, int precision, bool batch, ResMode& M) {
     std::vector<size_t> at_rows(nseg), at_split(nseg);
     for (int i = 0; i < nseg; ++i) {
       const int n0 = c->h_seg_node[i], n1 = c->h_seg_node[i + 1];
+      if (n0 == n1) return TG_OK;  // an RVE without nodes: refused by the streamed solve
       resident_rows(n0, n1, c->h_rowptr.data(), c->h_col.data(), mask.data(), rows[i]);
       ResPlan P;
       if (!rows[i].act_node.empty() && !resident_plan(rows[i], elem, c->num_sms, limits, false, P)) return TG_OK;
