@@ -62,7 +62,7 @@ struct ResPlan {
   std::vector<int> part_chunk;
   std::vector<int4> part_win;
   ResPlanDev dev{};
-  void* buf = nullptr;  // device copy of the split
+  int elem0 = 0;        // element that its contribution map counts from
 };
 
 // The plans of the current mesh for one precision, for a solve of the whole
