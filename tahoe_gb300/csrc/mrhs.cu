@@ -627,6 +627,7 @@ int macro_tangent_mrhs(Context* c, int precision, int precond, double rel_tol, i
   if (c->seg_pcg_mode && ke_current(c)) {
     const int sr = resident_active(c, precision, &resident);
     if (sr) return sr;
+    resident = resident && resident_whole(c, precision);
   }
   if (!resident) {
     const int sf = ensure_full_assembly(c);

@@ -465,6 +465,13 @@ int push_prepare(Context* c, int precision) {
   if (s) return s;
   long long& serial = f32 ? ps.serial32 : ps.serial64;
   if (serial == c->tangent_serial) return TG_OK;
+  if ((f32 ? c->full_serial32 : c->full_serial64) != c->tangent_serial && precision == c->tangent_precision &&
+      (f32 ? c->ke_serial32 : c->ke_serial64) >= 0) {
+    // a tangent without a storage: straight from its element blocks
+    s = launch_assemble_upper(c, precision);
+    if (!s) serial = c->tangent_serial;
+    return s;
+  }
   // copied from the full storage (assembled there for another solve)
   s = ensure_full_assembly(c);
   if (s) return s;

@@ -1163,9 +1163,8 @@ int plan_rows(Context* c, int precision, bool batch, ResMode& M) {
         bool fits = false;
         s = template_resident(c, t, precision, P, fits);
         if (s) return s;
-        if (!fits) return TG_OK;
-        it = seen.emplace(t, (int)M.plans.size()).first;
-        M.plans.push_back(P);
+        it = seen.emplace(t, fits ? (int)M.plans.size() : -1).first;
+        if (fits) M.plans.push_back(P);
       }
       M.plan_of.push_back(it->second);
     }
@@ -1243,8 +1242,10 @@ int plan_rows(Context* c, int precision, bool batch, ResMode& M) {
     });
     ResImage blocks, img;  // every plan's blocks, then the rest
     std::vector<size_t> at_blk(np), at_rows(np), at_split(np);
+    std::vector<int> kept(np, -1);
     for (int p = 0; p < np; ++p) {
-      if (!fits[p]) return TG_OK;
+      if (!fits[p]) continue;
+      kept[p] = (int)M.plans.size();
       ResPlan& P = plans[p];
       at_blk[p] = blocks.data.size();
       blocks.data.insert(blocks.data.end(), rows[p].blk.begin(), rows[p].blk.end());
@@ -1254,6 +1255,7 @@ int plan_rows(Context* c, int precision, bool batch, ResMode& M) {
       P.elem0 = c->h_seg_elem[first[p]];
       M.plans.push_back(P);
     }
+    for (int& p : M.plan_of) p = kept[p];
     int *d = nullptr, *blk = nullptr;
     int2* slot = nullptr;
     if (!hold(c, M, &d, img.data.size()) || !hold(c, M, &slot, blocks.data.size()) ||
@@ -1271,14 +1273,18 @@ int plan_rows(Context* c, int precision, bool batch, ResMode& M) {
     dfree(c, blk);  // the slots name their contributions
     if (s) return s;
     for (int p = 0; p < np; ++p) {
-      ResPlanDev& D = M.plans[p].dev;
+      if (kept[p] < 0) continue;
+      ResPlan& P = M.plans[kept[p]];
+      ResPlanDev& D = P.dev;
       resident_bind_rows(D, d, at_rows[p], rows[p]);
-      resident_bind_split(D, d, at_split[p], M.plans[p]);
+      resident_bind_split(D, d, at_split[p], P);
       D.blk = nullptr;
       D.slot = slot + at_blk[p];
       D.contrib = c->d_contrib;
     }
   }
+  for (int p : M.plan_of) M.streamed += p < 0 ? 1 : 0;
+  if (M.plans.empty()) return TG_OK;
   std::vector<ResPlanDev> dev;
   for (const ResPlan& P : M.plans) dev.push_back(P.dev);
   if (!hold(c, M, &M.d_plans, std::max<size_t>(dev.size(), 1))) return TG_ERR_OOM;
@@ -1347,11 +1353,11 @@ struct AuxStreams {
 
 // Runs the solves of the listed RVEs (act; one for a whole mesh) for nvec
 // right-hand sides, nnd nodes apart in d_rhs and x, and reports each in out.
-// x is zero away from the solved rows.
+// x is zero away from the solved rows; with keep_x they stay as they are.
 template <typename T>
 int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>& act, const double4_32a* d_rhs, int nvec,
                  typename Vec4<T>::type* x, double rel_tol, int max_it, int precond, std::vector<ResItem>& items,
-                 std::vector<ResOut>& out) {
+                 std::vector<ResOut>& out, bool keep_x = false) {
   using V = typename Vec4<T>::type;
   ResState& S = *c->res;
   int s = TG_OK;
@@ -1366,8 +1372,8 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
   };
   std::map<std::vector<long long>, Class> cls;
   for (int i = 0; i < nseg; ++i) {
+    if (!act[i] || M.plan_of[i] < 0 || M.plans[M.plan_of[i]].rows == 0) continue;
     const ResPlan& P = M.plans[M.plan_of[i]];
-    if (!act[i] || P.rows == 0) continue;
     const long long b = (long long)((P.smem + 16383) / 16384);
     Class& C = cls[{P.grid ? 0 : 1, -(long long)P.k, -P.warps, P.one ? 1 : 0, -b}];
     C.grid = P.grid;
@@ -1401,7 +1407,7 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
     if (s) return s;
   }
   // rows outside every solve (prescribed nodes, RVEs not solved) stay zero
-  if (!ok(c, cudaMemsetAsync(x, 0, sizeof(V) * (size_t)c->nnd * nvec, st), "x") ||
+  if ((!keep_x && !ok(c, cudaMemsetAsync(x, 0, sizeof(V) * (size_t)c->nnd * nvec, st), "x")) ||
       !ok(c, cudaMemsetAsync(S.d_out, 0, sizeof(ResOut) * (size_t)std::max(n, 1), st), "out"))
     return TG_ERR_CUDA;
   if (n == 0) {
@@ -1499,9 +1505,36 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
   const int nseg = batch ? c->nseg : 1;
   std::vector<uint8_t> act(nseg, 1);
   if (batch && (int)c->seg_active.size() == nseg) act = c->seg_active;
+  // RVEs that do not fit: the streamed per-RVE solve first, which sets the
+  // others' rows to zero; an RVE takes the same solve in every batch
+  int worst_it = 0;
+  double worst_rel = 0.0;
+  bool streamed = false;
+  if (batch && M.streamed > 0) {
+    std::vector<uint8_t> sub(act);
+    for (int i = 0; i < nseg; ++i) {
+      if (M.plan_of[i] >= 0) sub[i] = 0;
+      streamed = streamed || sub[i];
+    }
+    if (streamed) {
+      const bool tolerate = c->seg_tolerate;
+      sub.swap(c->seg_active);
+      c->seg_tolerate = true;
+      s = push_solve(c) ? push_prepare(c, c->tangent_precision) : ensure_full_assembly(c);
+      if (!s) {
+        std::memset(c->h_pcg, 0, sizeof(PcgScalars));
+        s = pcg_solve_segmented(c, d_rhs, rel_tol, max_it, precond, &worst_it, &worst_rel);
+        // what single RVEs came to is in seg_status
+        if ((s == TG_ERR_NAN && c->h_pcg[0].fail != 5) || s == TG_ERR_NOT_CONVERGED) s = TG_OK;
+      }
+      sub.swap(c->seg_active);
+      c->seg_tolerate = tolerate;
+      if (s) return s;
+    }
+  }
   std::vector<ResItem> items;
   std::vector<ResOut> out;
-  s = run_resident<T>(c, M, batch, act, d_rhs, 1, (V*)c->d_x, rel_tol, max_it, precond, items, out);
+  s = run_resident<T>(c, M, batch, act, d_rhs, 1, (V*)c->d_x, rel_tol, max_it, precond, items, out, streamed);
   if (s) return s;
   const int n = (int)items.size();
   if (!batch) {
@@ -1519,22 +1552,20 @@ int solve_resident_t(Context* c, ResMode& M, const double4_32a* d_rhs, double re
     return pcg_finish(c, h, iters, rel_res);
   }
   c->have_du = true;
-  int worst_it = 0, broke = 0, limit = 0, nact = 0, timeout = 0;
-  double worst_rel = 0.0;
-  c->seg_status.assign(nseg, TG_OK);
-  for (uint8_t a : act) nact += a ? 1 : 0;
+  int broke = 0, limit = 0, nact = 0, timeout = 0;
+  if (!streamed) c->seg_status.assign(nseg, TG_OK);
   for (int i = 0; i < n; ++i) {
     const ResOut& o = out[i];
     worst_it = std::max(worst_it, o.iters);
     if (o.rr0 > 0.0) worst_rel = std::max(worst_rel, std::sqrt(o.rr / o.rr0));
-    if (o.done == 2) {
-      c->seg_status[items[i].seg] = TG_ERR_NAN;
-      ++broke;
-      timeout += o.fail == 5 ? 1 : 0;
-    } else if (o.done != 1) {
-      c->seg_status[items[i].seg] = TG_ERR_NOT_CONVERGED;
-      ++limit;
-    }
+    c->seg_status[items[i].seg] = o.done == 2 ? TG_ERR_NAN : o.done != 1 ? TG_ERR_NOT_CONVERGED : TG_OK;
+    timeout += o.done == 2 && o.fail == 5 ? 1 : 0;
+  }
+  for (int i = 0; i < nseg; ++i) {
+    if (!act[i]) continue;
+    ++nact;
+    broke += c->seg_status[i] == TG_ERR_NAN ? 1 : 0;
+    limit += c->seg_status[i] == TG_ERR_NOT_CONVERGED ? 1 : 0;
   }
   if (iters) *iters = worst_it;
   if (rel_res) *rel_res = worst_rel;
@@ -1638,6 +1669,11 @@ int resident_active(Context* c, int precision, bool* on) {
   }
   *on = M.state > 0;
   return TG_OK;
+}
+
+// Whether a batch's every RVE is solved on the chip.
+bool resident_whole(const Context* c, int precision) {
+  return c->res->mode[precision == TG_MIXED ? 1 : 0][1].streamed == 0;
 }
 
 // The mode of the next solve of a precision, given up: a solve found no room for

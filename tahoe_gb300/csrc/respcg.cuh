@@ -70,7 +70,8 @@ struct ResPlan {
 struct ResMode {
   int state = 0;  // 0 not planned, 1 resident, 2 hybrid, -1 neither
   std::vector<ResPlan> plans;
-  std::vector<int> plan_of;  // plan of every RVE (one entry for a whole mesh)
+  std::vector<int> plan_of;  // plan of every RVE (one entry for a whole mesh), -1: streamed
+  int streamed = 0;          // RVEs that do not fit
   ResPlanDev* d_plans = nullptr;
   std::vector<void*> bufs;   // its device buffers
 };

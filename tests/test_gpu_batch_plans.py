@@ -58,3 +58,63 @@ def test_uploaded_rves_with_and_without_a_common_plan(precision, rel_tol, bound)
         c.tangent(precision)
         du[form] = c.pcg(None, rel_tol=rel_tol, max_it=2000)[0]
     assert np.abs(du[-1] - du[3]).max() < bound * np.abs(du[3]).max()
+
+
+@pytest.mark.parametrize("precision,side", [(lib.FP64, 33), (lib.MIXED, 46)])
+@pytest.mark.parametrize("composed", [False, True])
+def test_an_rve_beside_one_that_does_not_fit(precision, side, composed):
+    """The large one is streamed, the others are solved on the chip: each as it
+    is alone, bitwise, updates and iterations."""
+    ns = [6, side, 9]
+    Fs = [np.eye(3) + 0.01 * rve.sample_F(np.random.default_rng(i)) for i in range(3)]
+
+    def solve(which):
+        if composed:
+            c = lib.Context(0)
+            r = rve.ResidentRVEs(c)
+            r.compose([ns[i] for i in which])
+            c.set_u(np.zeros((c.nnd, 3)))
+            c.set_affine(np.array([Fs[i] for i in which]))
+        else:
+            b = rve.RVEBatch([ns[i] for i in which], [Fs[i] for i in which])
+            c = b.setup()
+            c.set_u(np.zeros((c.nnd, 3)))
+            c.set_prescribed(b.prescribed_idx, b.prescribed_val)
+        c.residual(want_vector=False)
+        c.tangent(precision)
+        its = c.pcg(None, rel_tol=1e-5, max_it=4000, want_du=False)[1]
+        c.apply_update()
+        u = c.get_u()
+        cut = np.concatenate([[0], np.cumsum([(ns[i] + 1) ** 3 for i in which])])
+        return its, [u[a:b] for a, b in zip(cut[:-1], cut[1:])]
+
+    its, u = solve([0, 1, 2])
+    alone = [solve([i]) for i in range(3)]
+    assert its == max(a[0] for a in alone)
+    for i in range(3):
+        assert np.abs(u[i]).max() > 0 and np.array_equal(u[i], alone[i][1][0]), ns[i]
+
+
+def test_failing_rves_beside_ones_that_do_not_fit():
+    """One Newton iteration with exact inner solves: RVEs under a tiny
+    deformation, which start at round-off, fail and the others converge.  Every
+    outcome and every converged stress is the RVE's own, alone (bitwise), for
+    the streamed ones and those on the chip."""
+    rng = np.random.default_rng(5)
+    S = [rve.sample_F(rng) - np.eye(3) for _ in range(4)]
+    ns = [4, 33, 5, 33]
+    Fs = [np.eye(3) + f * S[i] for i, f in enumerate((2e-5, 2e-5, 1.0, 0.02))]
+    kw = dict(precision=lib.FP64, rel_tol=1e-8, lin_rel_tol=1e-12, max_iterations=1)
+    alone = []
+    for i in range(4):
+        b = rve.RVEBatch(ns[i:i + 1], Fs[i:i + 1])
+        P = b.solve(**kw)[3]
+        alone.append((int(b.status[0]), P[0]))
+    b = rve.RVEBatch(ns, Fs)
+    rc, rep, rel, P = b.solve(**kw)
+    st = [int(v) for v in b.status]
+    assert st == [a[0] for a in alone]
+    assert 0 in st and rc == next(v for v in st if v != 0)
+    for i in range(4):
+        if st[i] == 0:
+            assert np.array_equal(P[i], alone[i][1]), i
