@@ -434,12 +434,32 @@ void drop_graphs(Context* c) {
 // by the assembly.
 int ensure_blob(Context* c, int precision) {
   unsigned char** blob = precision == TG_MIXED ? &c->d_blob32 : &c->d_blob64;
-  if (*blob) return TG_OK;
+  bool& ready = precision == TG_MIXED ? c->blob_ready32 : c->blob_ready64;
+  if (*blob && ready) return TG_OK;
   const std::vector<long long>& off = precision == TG_MIXED ? c->h_blob_off32 : c->h_blob_off64;
   const long long total = off[c->ntiles];
-  if (!dalloc(c, blob, (size_t)total)) return TG_ERR_OOM;
+  if (!*blob && !dalloc(c, blob, (size_t)total)) return TG_ERR_OOM;
+  ready = false;
   if (!ok(c, cudaMemsetAsync(*blob, 0, (size_t)total, c->stream), "blob")) return TG_ERR_CUDA;
-  return launch_blob_structure(c, precision);
+  const int s = launch_blob_structure(c, precision);
+  ready = s == TG_OK;
+  return s;
+}
+
+// The storage's bytes alone, for tg_pcg_solve_noalloc after a tangent whose own
+// solve needs none.  Without room for them that call will find none.
+void reserve_blob(Context* c, int precision) {
+  unsigned char** blob = precision == TG_MIXED ? &c->d_blob32 : &c->d_blob64;
+  if (*blob || c->nnd > kNoAllocMaxNodes) return;
+  const size_t total = (size_t)(precision == TG_MIXED ? c->h_blob_off32 : c->h_blob_off64)[c->ntiles];
+  void* p = nullptr;
+  if (cudaMallocAsync(&p, std::max<size_t>(total, 1), c->stream) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  c->allocations.push_back(p);
+  *blob = (unsigned char*)p;
+  (precision == TG_MIXED ? c->blob_ready32 : c->blob_ready64) = false;
 }
 }  // namespace tg
 

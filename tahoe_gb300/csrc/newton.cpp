@@ -117,6 +117,7 @@ int form_tangent(Context* c, int precision) {
   const bool push = !resident && push_solve(c);
   if (!s && !resident) s = push ? push_structure(c, precision) : ensure_blob(c, precision);
   if (s) return s;
+  if (resident && !push_solve(c)) reserve_blob(c, precision);
   (precision == TG_MIXED ? c->ke_serial32 : c->ke_serial64) = -1;
   s = launch_tangent(c, precision);
   if (!s && resident) {

@@ -15,7 +15,7 @@
 
 namespace {
 
-constexpr int kNoAllocMaxNodes = 32768;
+using tg::kNoAllocMaxNodes;
 constexpr size_t kNoAllocScratchBytes = 8u << 20;  // 8 MiB per device
 static_assert(tg::kScratchScalarBytes + tg::kScratchPartialBytes + (32 + 5 * 32) * (size_t)kNoAllocMaxNodes <=
                   kNoAllocScratchBytes,

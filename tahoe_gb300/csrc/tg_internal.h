@@ -262,6 +262,7 @@ struct Context {
   // one sequential range.
   unsigned char* d_blob32 = nullptr;
   unsigned char* d_blob64 = nullptr;
+  bool blob_ready32 = false, blob_ready64 = false;  // structure written
   long long* d_blob_off32 = nullptr;  // ntiles+1
   long long* d_blob_off64 = nullptr;
   std::vector<long long> h_blob_off32, h_blob_off64;
@@ -393,6 +394,8 @@ int build_tiles(Context* c, int tile_blocks);
 int spmv_grid_for(Context* c, long long cap32);
 void drop_graphs(Context* c);  // captured Krylov iterations (their launches bake in the product's shape)
 int ensure_blob(Context* c, int precision);
+void reserve_blob(Context* c, int precision);
+constexpr int kNoAllocMaxNodes = 32768;  // of tg_pcg_solve_noalloc
 
 // blob geometry shared by host and device code
 __host__ __device__ inline int ceil4(int n) { return (n + 3) & ~3; }

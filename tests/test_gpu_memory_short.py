@@ -34,12 +34,12 @@ def _solve(c):
     return c.pcg(None, rel_tol=1e-6, max_it=2000)[0]
 
 
-@pytest.mark.parametrize("precision", [lib.FP64, lib.MIXED])
-@pytest.mark.parametrize("form", [1, 3])
-def test_tangent_without_room_leaves_the_last_one(precision, form):
+@pytest.mark.parametrize("precision,form,n", [(lib.FP64, 3, 16), (lib.MIXED, 3, 16), (lib.MIXED, 1, 33)])
+def test_tangent_without_room_leaves_the_last_one(precision, form, n):
     """The default form solves this mesh without a matrix storage; the streamed
-    form's storage then finds no room, at another displacement."""
-    c, mesh = _context()
+    form's storage then finds no room, at another displacement.  (Form 1's bytes
+    are reserved on meshes of up to 32,768 nodes.)"""
+    c, mesh = _context(n)
     c.tangent(precision)
     ref = _solve(c)
     c.set_u(0.02 * mesh.X * np.array([1.0, -0.3, 0.2]))
