@@ -425,6 +425,14 @@ int tg_pcg_form(tg_context* ctx, int form);
 /* the streamed form of the next single-vector solve on the current mesh
  * (0..3); with form -1 the one it takes where it does not solve on the chip */
 int tg_pcg_form_get(const tg_context* ctx, int* form);
+/* where the next solve and tangent of a precision run (either pointer may be
+ * NULL; plans the mesh if no solve did).  pcg: TG_ROUTE_STREAMED in the form
+ * above, TG_ROUTE_CHIP on the chip, TG_ROUTE_HYBRID the same with part of the
+ * matrix read from L2 and memory, TG_ROUTE_SOME a batch with RVEs of either
+ * kind.  general_tangent: 1 if the element matrices come from the general
+ * kernel, whose shape tg_tangent_config sets. */
+enum { TG_ROUTE_STREAMED = 0, TG_ROUTE_CHIP = 1, TG_ROUTE_HYBRID = 2, TG_ROUTE_SOME = 3 };
+int tg_routes_get(tg_context* ctx, int precision, int* pcg, int* general_tangent);
 /* L2 priorities of the streamed matrix.  bytes >= 0: the leading whole
  * tiles within `bytes` of the matrix storage are copied with evict_last
  * (kept in the L2 from one product to the next) and the rest with

@@ -507,6 +507,14 @@ int tg_pcg_form_get(const tg_context* c, int* form) {
   return TG_OK;
 }
 
+int tg_routes_get(tg_context* c, int precision, int* pcg, int* general_tangent) {
+  if (!c || c->nnd <= 0 || (precision != TG_FP64 && precision != TG_MIXED)) return TG_ERR_ARG;
+  if (set_device(c)) return TG_ERR_CUDA;
+  if (general_tangent)
+    *general_tangent = !tangent_iso_applies(c, precision) && !tangent_blocks_applies(c, precision) ? 1 : 0;
+  return pcg ? resident_route(c, precision, pcg) : TG_OK;
+}
+
 int tg_spmv_l2_keep(tg_context* c, long long bytes) {
   if (!c || bytes < -1) return TG_ERR_ARG;
   c->l2_keep = bytes;

@@ -1671,6 +1671,16 @@ int resident_active(Context* c, int precision, bool* on) {
   return TG_OK;
 }
 
+int resident_route(Context* c, int precision, int* route) {
+  bool on = false;
+  const int s = resident_active(c, precision, &on);
+  *route = TG_ROUTE_STREAMED;
+  if (s || !on) return s;
+  const ResMode& M = c->res->mode[precision == TG_MIXED ? 1 : 0][c->nseg > 0 && c->seg_pcg_mode ? 1 : 0];
+  *route = M.state == 2 ? TG_ROUTE_HYBRID : M.streamed > 0 ? TG_ROUTE_SOME : TG_ROUTE_CHIP;
+  return TG_OK;
+}
+
 // Whether a batch's every RVE is solved on the chip.
 bool resident_whole(const Context* c, int precision) {
   return c->res->mode[precision == TG_MIXED ? 1 : 0][1].streamed == 0;

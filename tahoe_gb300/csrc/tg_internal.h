@@ -507,6 +507,7 @@ void cg_free(Context* c);  // the captured iterations
 int resident_active(Context* c, int precision, bool* on);
 void resident_refuse(Context* c, int precision);
 bool resident_whole(const Context* c, int precision);
+int resident_route(Context* c, int precision, int* route);  // TG_ROUTE_*
 int pcg_solve_resident(Context* c, const double4_32a* d_rhs, double rel_tol, int max_it, int precond, int* iters,
                        double* rel_res);
 // nvec right-hand sides of every RVE of a batch: w = v + K^-1 b per RVE

@@ -95,6 +95,7 @@ _SIGS = {
     "tg_spmv_l2_keep": (ctypes.c_int, [_vp, ctypes.c_longlong]),
     "tg_pcg_form": (ctypes.c_int, [_vp, ctypes.c_int]),
     "tg_pcg_form_get": (ctypes.c_int, [_vp, _ip]),
+    "tg_routes_get": (ctypes.c_int, [_vp, ctypes.c_int, _ip, _ip]),
     "tg_tuning_get": (ctypes.c_int, [_vp, _ip, _ip, _ip]),
     "tg_set_segments": (ctypes.c_int, [_vp, ctypes.c_int, _ip, _ip]),
     "tg_segment_residual_norms": (ctypes.c_int, [_vp, _dp]),
@@ -521,6 +522,15 @@ class Context:
         f = ctypes.c_int(0)
         self._chk(self.L.tg_pcg_form_get(self.h, ctypes.byref(f)), "tg_pcg_form_get")
         return f.value
+
+    def routes(self, precision):
+        """Where the next solve and tangent of a precision run: (route,
+        general), route "streamed" (in effective_form()), "chip", "hybrid" or
+        "some" (a batch with RVEs of either kind), general whether the element
+        matrices come from the kernel whose shape tangent_config() sets."""
+        p, g = ctypes.c_int(0), ctypes.c_int(0)
+        self._chk(self.L.tg_routes_get(self.h, int(precision), ctypes.byref(p), ctypes.byref(g)), "tg_routes_get")
+        return ("streamed", "chip", "hybrid", "some")[p.value], bool(g.value)
 
     def spmv_l2_keep(self, nbytes):
         """Matrix bytes the streamed product keeps in the L2 (evict_last;
