@@ -10,13 +10,16 @@ themselves (CUDA events, tg_time_kernel) on the current state:
     x upper blocks per tile), which replaces the full storage where it is
     faster on the mesh at hand;
   * the element tangent: elements per CTA (one thread per upper node-pair
-    block of each element).
+    block of each element), where the general kernel forms it.
 
-When the solve streams the symmetric push storage (tg_pcg_form 3, the
-default on meshes of a million block nonzeros and more), the product has
-the one launch shape of that storage: the full-storage and symmetric-format
-sweeps are skipped (they would time the same product for every candidate)
-and only the tangent is tuned.
+When the solve runs on the chip (tg_routes_get; the default form on most
+meshes), no streamed product runs: nothing about one is tuned, and the
+symmetric format, which would take the mesh off the chip, stays off.  When
+the solve streams the symmetric push storage (tg_pcg_form 3, the default on
+meshes of a million block nonzeros and more that do not fit the chip), the
+product has the one launch shape of that storage: the full-storage and
+symmetric-format sweeps are skipped (they would time the same product for
+every candidate).  In both only the tangent is tuned.
 
 Results are cached per (GPU, precision, formulation, mesh-size bucket) in a
 JSON table, so a serving process tunes once per kind of mesh.  Element
@@ -43,12 +46,29 @@ _DEFAULT_CACHE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_buil
 
 def signature(ctx, precision, formulation, gpu="gpu0"):
     """Cache key: mesh sizes bucketed to powers of two (shapes are chosen for
-    the size class, not the exact mesh), and whether the solve streams the
-    push storage."""
+    the size class, not the exact mesh), whether the solve runs on the chip,
+    streams the push storage or streams while the other precision's runs on the
+    chip, and whether the general kernel forms the tangent."""
     b = lambda x: 1 << max(0, int(math.log2(max(1, x))))
+    chip, general = _routes(ctx, precision)
     form = getattr(ctx, "effective_form", None)
-    push = "|push" if form is not None and form() == 3 else ""
-    return "%s|p%d|f%d|nnd%d|nel%d%s" % (gpu, precision, formulation, b(ctx.nnd), b(ctx.nel), push)
+    other = _routes(ctx, _other(precision))[0]
+    kind = "|chip" if chip else "|push" if form is not None and form() == 3 else "|beside" if other else ""
+    return "%s|p%d|f%d|nnd%d|nel%d%s%s" % (gpu, precision, formulation, b(ctx.nnd), b(ctx.nel), kind,
+                                           "" if general else "|own")
+
+
+def _other(precision):
+    return lib.MIXED if precision == lib.FP64 else lib.FP64
+
+
+def _routes(ctx, precision):
+    """(the solve runs on the chip, the general kernel forms the tangent)"""
+    routes = getattr(ctx, "routes", None)
+    if routes is None:
+        return False, True
+    route, general = routes(precision)
+    return route != "streamed", general
 
 
 def pick(timings):
@@ -86,7 +106,7 @@ class Tuner:
 
     @staticmethod
     def apply(ctx, cfg):
-        if cfg.get("push"):  # the push storage's product keeps its one shape
+        if cfg.get("push") or cfg.get("chip"):  # no product with a shape to choose
             ctx.tangent_config(cfg["tangent_epb"])
             return
         ctx.spmv_config(cfg["tile_blocks"], cfg["stages"])
@@ -105,9 +125,10 @@ class Tuner:
             self.apply(ctx, cfg)
             return dict(cfg, cached=True)
         timer = timer or (lambda c, which, reps: c.time_kernel(which, reps))
+        chip, general = _routes(ctx, precision)
         form = getattr(ctx, "effective_form", None)
-        if form is not None and form() == 3:
-            return self._tune_tangent_only(ctx, precision, key, timer)
+        if chip or (form is not None and form() == 3):
+            return self._tune_tangent_only(ctx, precision, key, timer, chip, general)
         spmv = {}
         for t in self.tiles:
             for s in self.stages:
@@ -132,9 +153,10 @@ class Tuner:
         ctx.spmv_config(tb, st)
         ctx.spmv_release(rl)
         ctx.tangent(precision)
-        # the symmetric stream format, against the best full-storage shape
+        # the symmetric stream format, against the best full-storage shape; not
+        # where it would take the other precision's solves off the chip
         sym = {}
-        for m in self.sym_modes:
+        for m in () if _routes(ctx, _other(precision))[0] else self.sym_modes:
             for t in self.sym_tiles:
                 try:
                     ctx.spmv_symmetric(m, t)
@@ -146,10 +168,7 @@ class Tuner:
         best_sym, sym_ms = pick(sym) if sym else (None, float("inf"))
         sm, stile = (best_sym if best_sym is not None and sym_ms < spmv_ms else (0, 0))
         ctx.spmv_symmetric(sm, stile)
-        tang = {}
-        for e in self.epbs:
-            ctx.tangent_config(e)
-            tang[e] = timer(ctx, KERNEL_TANGENT, max(3, self.reps // 4))
+        tang = self._tangent_sweep(ctx, timer, general)
         epb, tang_ms = pick(tang)
         cfg = {"tile_blocks": tb, "stages": st, "release": rl, "sym": sm, "sym_tile": stile, "tangent_epb": epb,
                "spmv_ms": min(spmv_ms, sym_ms) if sm else spmv_ms, "tangent_ms": tang_ms}
@@ -163,20 +182,29 @@ class Tuner:
         out["tangent_sweep"] = {str(k): v for k, v in tang.items()}
         return out
 
-    def _tune_tangent_only(self, ctx, precision, key, timer):
-        """The push storage's solve: the product keeps its one shape (timed
-        for the record), the tangent's elements per CTA are tuned."""
-        cur = ctx.tuning()
-        ctx.tangent(precision)
-        spmv_ms = timer(ctx, KERNEL_SPMV, self.reps)
+    def _tangent_sweep(self, ctx, timer, general):
+        """{elements per CTA: ms}; the present one alone where another kernel,
+        without that choice, forms the tangent."""
         tang = {}
-        for e in self.epbs:
+        for e in self.epbs if general else (ctx.tuning()["tangent_epb"],):
             ctx.tangent_config(e)
             tang[e] = timer(ctx, KERNEL_TANGENT, max(3, self.reps // 4))
+        return tang
+
+    def _tune_tangent_only(self, ctx, precision, key, timer, chip, general):
+        """A solve on the chip, or the push storage's: its product keeps its
+        one shape (the streamed one is timed for the record), the tangent's
+        elements per CTA are tuned."""
+        cur = ctx.tuning()
+        ctx.tangent(precision)
+        spmv_ms = None if chip else timer(ctx, KERNEL_SPMV, self.reps)
+        tang = self._tangent_sweep(ctx, timer, general)
         epb, tang_ms = pick(tang)
         cfg = {"tile_blocks": cur["tile_blocks"], "stages": cur["stages"], "release": 0, "sym": 0, "sym_tile": 0,
-               "tangent_epb": epb, "spmv_ms": spmv_ms, "tangent_ms": tang_ms, "push": True}
+               "tangent_epb": epb, "spmv_ms": spmv_ms, "tangent_ms": tang_ms}
+        cfg["chip" if chip else "push"] = True
         ctx.tangent_config(epb)
+        ctx.tangent(precision)  # the timing overwrote its element blocks
         self.table[key] = cfg
         self.save()
         out = dict(cfg, cached=False)

@@ -122,3 +122,31 @@ def test_push_storage_tunes_the_tangent_only(tmp_path):
     assert autotune.signature(ctx, lib.MIXED, lib.TOTAL_LAGRANGIAN) != \
         autotune.signature(FakeCtx(), lib.MIXED, lib.TOTAL_LAGRANGIAN)
 
+
+
+class FakeChipCtx(FakePushCtx):
+    """A context whose solve runs on the chip."""
+
+    def __init__(self, general, **kw):
+        super().__init__(**kw)
+        self.general = general
+
+    def effective_form(self):
+        return 1
+
+    def routes(self, precision):
+        return "chip", self.general
+
+
+def test_solve_on_the_chip_tunes_no_product(tmp_path):
+    def timer(ctx, which, reps):
+        assert which == autotune.KERNEL_TANGENT
+        return fake_timer(ctx, which, reps)
+
+    for general, epb in ((True, 4), (False, 8)):
+        ctx = FakeChipCtx(general)
+        out = autotune.Tuner(cache_path=str(tmp_path / "t.json"), reps=4).tune(ctx, lib.MIXED, lib.SMALL_STRAIN,
+                                                                              timer=timer)
+        assert out["chip"] and not out["cached"] and out["sym"] == 0 and out["spmv_ms"] is None
+        assert out["tangent_epb"] == ctx.cfg["tangent_epb"] == epb
+        assert len(out["tangent_sweep"]) == (3 if general else 1)
