@@ -507,6 +507,14 @@ int tg_pcg_form_get(const tg_context* c, int* form) {
   return TG_OK;
 }
 
+// For tests: the limits of the waits in the solves on the chip.
+int tgx_wait_limits(tg_context* c, int polls, int mute) {
+  if (!c || polls < 64) return TG_ERR_ARG;
+  c->waits.polls = polls;
+  c->waits.mute = mute;
+  return TG_OK;
+}
+
 int tg_routes_get(tg_context* c, int precision, int* pcg, int* general_tangent) {
   if (!c || c->nnd <= 0 || (precision != TG_FP64 && precision != TG_MIXED)) return TG_ERR_ARG;
   if (set_device(c)) return TG_ERR_CUDA;

@@ -74,6 +74,7 @@ struct HybArgs {
   ResOut* out;
   PcgScalars* sc;
   int* status;
+  WaitLimits waits;
   long long chunks;
   int rows, uwcap, chcap; // shared memory: window rows, chunks
   int in_smem;            // of p, s, preconditioner: how many are in shared memory
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(kHybWarps * 32, 1) hybrid_kernel(HybArgs A) {
     AccMax mx[3];
     for (int i = warp; i < nch; i += kHybWarps) mx[0].v = max(mx[0].v, exponent_of(rhs_at(i)));
     ++seq;
-    total3<AccMax, float, true>(mx, sh, k, rank, seq, inbox);
+    total3<AccMax, float, true>(mx, sh, k, rank, seq, inbox, A.waits);
     __syncthreads();
     const int e1 = (int)sh.tot[0];
     if (e1 > 0 && e1 < 0x7ff) scale_exp = max(-1000, min(1000, 1023 - e1));
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(kHybWarps * 32, 1) hybrid_kernel(HybArgs A) {
     }
     __syncthreads();
     ++seq;
-    total3<AccMax, float, true>(mx, sh, k, rank, seq, inbox);
+    total3<AccMax, float, true>(mx, sh, k, rank, seq, inbox, A.waits);
     __syncthreads();
     const int e2 = (int)sh.tot[0];
     if (e2 > 0 && e2 < 0x7ff && e1 > 0 && e1 < 0x7ff) scale_exp = max(-1000, min(1000, scale_exp - (e2 - 1023) / 2));
@@ -277,11 +278,8 @@ __global__ void __launch_bounds__(kHybWarps * 32, 1) hybrid_kernel(HybArgs A) {
       const uint4* w = urow + halo[h];
       float x0, x1, x2;
       int tries = 0;
-      while (!RowWords<float>::load(w, (unsigned)it + 1u, x0, x1, x2))
-        if (++tries >= kResPollLimit) {
-          sh.abort_flag = 1;
-          break;
-        }
+      while (!RowWords<float>::load(w, (unsigned)it + 1u, x0, x1, x2) && poll_again(sh, A.waits, tries)) {
+      }
       uw[nown + h] = make_float4(x0, x1, x2, 0.f);
     }
     __syncthreads();
@@ -338,7 +336,7 @@ __global__ void __launch_bounds__(kHybWarps * 32, 1) hybrid_kernel(HybArgs A) {
       a[0].add_prod(u, w);
     }
     ++seq;
-    total3<Acc<float>, float, true>(a, sh, k, rank, seq, inbox);
+    total3<Acc<float>, float, true>(a, sh, k, rank, seq, inbox, A.waits);
     if (threadIdx.x == 0) scalars(sh, it, A.max_it, A.tol);
     __syncthreads();
     if (sh.code) break;
@@ -803,6 +801,7 @@ int hybrid_solve(Context* c, const double4_32a* d_rhs, double rel_tol, int max_i
   const int blk = precond == TG_PRECOND_BLOCK_JACOBI ? 1 : 0;
   HybArgs A = H.A;
   A.Ke = c->d_Ke32;
+  A.waits = c->waits;
   A.rhs = d_rhs;
   A.x = (float4*)c->d_x;
   A.sc = c->d_pcg;

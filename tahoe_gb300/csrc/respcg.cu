@@ -298,7 +298,7 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
       a[0].v = max(a[0].v, exponent_of(b[q]));
     }
     ++seq;
-    total3<AccMax, T, GRID>(a, sh, k, rank, seq, inbox);
+    total3<AccMax, T, GRID>(a, sh, k, rank, seq, inbox, A.waits);
     __syncthreads();
     const int e1 = (int)sh.tot[0];
     if (e1 > 0 && e1 < 0x7ff) scale_exp = max(-1000, min(1000, 1023 - e1));
@@ -312,7 +312,7 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
     }
     __syncthreads();  // sh.tot and sh.red are read
     ++seq;
-    total3<AccMax, T, GRID>(a, sh, k, rank, seq, inbox);
+    total3<AccMax, T, GRID>(a, sh, k, rank, seq, inbox, A.waits);
     __syncthreads();
     const int e2 = (int)sh.tot[0];
     if (e2 > 0 && e2 < 0x7ff && e1 > 0 && e1 < 0x7ff) scale_exp = max(-1000, min(1000, scale_exp - (e2 - 1023) / 2));
@@ -369,11 +369,8 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
         const uint4* w = urow + (size_t)(win.x + at) * RowWords<T>::n;
         T x0, x1, x2;
         int tries = 0;
-        while (!RowWords<T>::load(w, (unsigned)it + 1u, x0, x1, x2))
-          if (++tries >= kResPollLimit) {
-            sh.abort_flag = 1;
-            break;
-          }
+        while (!RowWords<T>::load(w, (unsigned)it + 1u, x0, x1, x2) && poll_again(sh, A.waits, tries)) {
+        }
         uw[at] = mk<V, T>(x0, x1, x2);
       }
       __syncthreads();
@@ -513,7 +510,7 @@ __device__ __forceinline__ void resident_solve(const ResArgs<T>& A, const ResIte
       }
     }
     ++seq;
-    total3<Acc<T>, T, GRID, !F32>(a, sh, k, rank, seq, inbox);
+    total3<Acc<T>, T, GRID, !F32>(a, sh, k, rank, seq, inbox, A.waits);
     if (threadIdx.x == 0) scalars(sh, it, A.max_it, A.tol);
     __syncthreads();
     if (sh.code) break;
@@ -1431,6 +1428,7 @@ int run_resident(Context* c, ResMode& M, bool batch, const std::vector<uint8_t>&
   A.ll = S.d_ll;
   A.sc = c->d_pcg;
   A.status = c->d_status;
+  A.waits = c->waits;
   A.batch = batch ? 1 : 0;
   const bool blk = precond == TG_PRECOND_BLOCK_JACOBI;
   A.max_it = max_it;

@@ -16,7 +16,6 @@ namespace {
 
 constexpr int kResClusterMax = 16;
 constexpr int kResCopies = 16;         // tables of the CTAs' sums (grid form)
-constexpr int kResPollLimit = 1 << 21;  // polls of one exchange word before the solve is abandoned
 
 // Shape of a CTA: warps, chunks of 8 rows per warp at most, and for a warp's
 // first `off` chunks the steps whose blocks stay out of shared memory.
@@ -217,6 +216,7 @@ struct ResArgs {
   uint4* ll;             // grid form: exchange words, zero before the launch
   PcgScalars* sc;        // receives unscale (single solve) or 1 (batch)
   int* status;
+  WaitLimits waits;
   int batch;             // the solution is unscaled in place
   int nnd;               // nodes of one right-hand side and solution
   int max_it;
@@ -242,6 +242,14 @@ struct ResShared {
   unsigned tmem;                     // the CTA's tensor memory
 };
 
+// After a poll of an exchange word that found it unwritten: whether to poll
+// again.  A wait that ran out ends the CTA's others within 64 polls.
+template <typename T>
+__device__ __forceinline__ bool poll_again(ResShared<T>& sh, const WaitLimits& W, int& tries) {
+  if (++tries >= W.polls) sh.abort_flag = 1;
+  return (tries & 63) != 0 || *reinterpret_cast<volatile int*>(&sh.abort_flag) == 0;
+}
+
 // Totals of three accumulators over every row of the solve, returned to
 // thread 0 (and left in sh.tot): lanes, warps and CTAs in a fixed order.  seq
 // numbers the reductions of a solve from 1.
@@ -253,7 +261,8 @@ struct ResShared {
 // one pass over shared memory.
 // ROWS: lane v of a row already holds the row's value v in a[0].
 template <typename A, typename T, bool GRID, bool ROWS = false>
-__device__ __forceinline__ void total3(A (&a)[3], ResShared<T>& sh, int k, int rank, unsigned seq, uint4* inbox) {
+__device__ __forceinline__ void total3(A (&a)[3], ResShared<T>& sh, int k, int rank, unsigned seq, uint4* inbox,
+                                       const WaitLimits& W) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (!ROWS)
 #pragma unroll
@@ -284,7 +293,7 @@ __device__ __forceinline__ void total3(A (&a)[3], ResShared<T>& sh, int k, int r
     asm volatile("bar.sync 1, %0;" ::"r"(np) : "memory");
     const u64 w0 = sh.tot[0], w1 = sh.tot[1], w2 = sh.tot[2];
     const u64 h0 = (w2 & 0xffffffffull) | ((u64)seq << 32), h1 = (w2 >> 32) | ((u64)seq << 32);
-    for (int q = threadIdx.x; q < copies; q += (int)np) {
+    for (int q = threadIdx.x; q < copies && rank != W.mute; q += (int)np) {
       uint4* w = inbox + (((size_t)q * 2 + par) * k + rank) * 2;
       st_word(w, w0, h0);
       st_word(w + 1, w1, h1);
@@ -298,11 +307,7 @@ __device__ __forceinline__ void total3(A (&a)[3], ResShared<T>& sh, int k, int r
       for (;;) {
         ld_word(w, x0, y0);
         ld_word(w + 1, x1, y1);
-        if (word_seq(y0) == seq && word_seq(y1) == seq) break;
-        if (++tries >= kResPollLimit) {
-          sh.abort_flag = 1;
-          break;
-        }
+        if ((word_seq(y0) == seq && word_seq(y1) == seq) || !poll_again(sh, W, tries)) break;
       }
       merge_word(g[0], x0);
       merge_word(g[1], x1);

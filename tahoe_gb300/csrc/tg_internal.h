@@ -71,6 +71,13 @@ struct ResidScalars {
   int pad;
 };
 
+// Limits of the waits in the solves on the chip: polls of one exchange word
+// (2^21: 1.5 s) before the solve is abandoned, after which its CTAs' other
+// waits end as well.  Tests set fewer, and a part whose sums are not sent.
+struct WaitLimits {
+  int polls = 1 << 21;
+  int mute = -1;
+};
 struct HybState;      // plan and buffers of the hybrid PCG (hybridpcg.cu)
 struct ResState;      // plans and buffers of the resident PCG (respcg.cuh)
 struct MeshTemplate;  // a resident template mesh (compose.cu)
@@ -250,6 +257,7 @@ struct Context {
   long long ke_serial32 = -1, ke_serial64 = -1;      // tangent serial of the element blocks on the device
   ResState* res = nullptr;
   HybState* hyb = nullptr;
+  WaitLimits waits;
   long long full_serial32 = -1, full_serial64 = -1;  // tangent serial of the full storage's values
   int* d_contrib_ptr = nullptr; // nnzb+1
   int* d_contrib = nullptr;     // nel*64: e*64 + a*8 + b
