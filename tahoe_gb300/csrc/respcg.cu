@@ -855,8 +855,9 @@ size_t part_bytes(const ResRows& R, int a, int b, int elem, int nw, int* lo, int
 }
 
 // The chunks cut into k consecutive parts of near-equal work; false if one
-// exceeds a CTA.
-bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
+// exceeds a CTA.  A CTA has a warp for each of its chunks (in fours), or all it
+// can have (full).
+bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P, bool full = false) {
   const int nch = (int)R.chunk_lo.size();
   if (k > nch) return false;
   const int warps = elem == 4 ? ResShape<float>::warps : ResShape<double>::warps;
@@ -887,7 +888,7 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
   for (int q = 0; q < k; ++q) most = std::max(most, P.part_chunk[q + 1] - P.part_chunk[q]);
   if (most > warps * slots) return false;
   // one chunk per warp while there are warps for it
-  P.warps = std::min(warps, (most + 3) / 4 * 4);
+  P.warps = full ? warps : std::min(warps, (most + 3) / 4 * 4);
   P.one = elem == 8 && most <= P.warps;
   for (int q = 0; q < k; ++q) {
     const int a = P.part_chunk[q], b = P.part_chunk[q + 1];
@@ -912,6 +913,8 @@ bool split_parts(const ResRows& R, int k, int elem, size_t cap, ResPlan& P) {
 }
 
 }  // namespace
+
+constexpr int kPollRows = 8;  // rows that a thread of the grid form polls
 
 // A split of the rows over CTAs.  A solve of a batch takes the fewest CTAs
 // that hold it (every SM has another RVE to solve), in FP64 as many more as
@@ -938,7 +941,33 @@ bool resident_plan(const ResRows& R, int elem, int num_sms, const ResLimits& L, 
     const int few = elem == 4 ? 24 : 4;
     P.grid = P.grid || (nch + max_cluster - 1) / max_cluster > few;
     const int k = std::max(kmin, std::min(nch, P.grid ? num_sms : max_cluster));
-    if (k != kmin && !split_parts(R, k, elem, cap, P) && !split_parts(R, kmin, elem, cap, P)) return false;
+    if (!P.grid) {
+      if (k != kmin && !split_parts(R, k, elem, cap, P) && !split_parts(R, kmin, elem, cap, P)) return false;
+    } else {
+      // Every thread polls its share of the other parts' rows in the window,
+      // 0.26 us a row: few where the nodes are numbered along the mesh, the
+      // whole mesh where they are not.  Above kPollRows a CTA has all its warps
+      // whatever its chunks (and in FP64 its tensor memory).  Shuffled numbers,
+      // streamed / a warp a chunk / all warps, us an iteration: FP32 4,913
+      // nodes 10.4 / 13.7 / 6.7, 9,261 10.8 / 14.1 / 9.7; FP64 5,832 21.7 / 26.2
+      // (the fewest CTAs that held it) / 15.5.
+      ResPlan best;
+      auto attempt = [&](bool full) {
+        ResPlan Q = P;
+        if (!split_parts(R, k, elem, cap, Q, full)) return false;
+        best = Q;
+        return true;
+      };
+      auto polls = [&]() {
+        int away = 0;
+        for (int q = 0; q < k; ++q)
+          away = std::max(away, best.part_win[q].y - (best.part_chunk[q + 1] - best.part_chunk[q]) * kResChunkRows);
+        return away / (32 * best.warps);
+      };
+      bool good = attempt(false);
+      if (!good || polls() > kPollRows) good = attempt(true) || good;
+      if (good) P = best;  // else the fewest CTAs
+    }
   } else if (!P.grid && elem == 8) {
     // the chip holds 15 clusters of 7, of 8 and of 9: in FP64, where a CTA's
     // time is that of its chunks, the largest costs nothing (48 RVEs with nine
