@@ -314,8 +314,10 @@ int tg_segment_solver(tg_context* ctx, int per_rve);
  * preconditioner, lin_rel_tol, lin_max_it) and dP = (1/V0) sum_a (K du)_a (x)
  * X_a.  C is nseg*81 doubles, C[s*81 + (3j+J)*9 + (3k+L)] = dP_jJ/dF_kL;
  * vol0 as for tg_segment_average_stress.  RVEs that the default
- * form solves on the chip (tg_pcg_form) take nine such solves each, every one
- * to lin_rel_tol of its own right-hand side.  Otherwise the nine solves run as
+ * form solves on the chip (tg_pcg_form; every RVE of the batch) take nine such
+ * solves each, every one to lin_rel_tol of its own right-hand side.  A solve
+ * that reaches lin_max_it first is not an error of this call: its column is
+ * what it had come to (*pcg_iterations is lin_max_it then).  Otherwise the nine solves run as
  * one multi-vector PCG over the whole batch: each right-hand side stops when its
  * residual norm over the batch falls below lin_rel_tol times its initial
  * norm over the batch (not per RVE), so an RVE's tangent in a batch agrees
