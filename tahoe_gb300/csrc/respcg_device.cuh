@@ -20,13 +20,17 @@ constexpr int kResCopies = 16;         // tables of the CTAs' sums (grid form)
 // Shape of a CTA: warps, chunks of 8 rows per warp at most, and for a warp's
 // first `off` chunks the steps whose blocks stay out of shared memory.
 //
-// FP32: 16 warps at 128 registers.  A warp's first chunk keeps seven steps (27
-// blocks a row) in registers, its second and third in tensor memory, the
-// fourth in shared memory, so a CTA holds 64 chunks where shared memory alone
+// FP32: 16 warps at 128 registers.  A warp's first chunk keeps four of its
+// seven steps (27 blocks a row) in registers, its second and third lie in
+// tensor memory, the rest in shared memory, so a CTA holds 64 chunks where shared memory alone
 // held 26: the SM's tensor memory is 256 KB that this solve's warps read
 // beside the shared-memory pipe (a step costs that pipe 5 wavefronts from
 // registers or tensor memory, its column indices and gathered vectors, and 14
-// from shared memory).  Fewer CTAs a solve also means more solves at once: a
+// from shared memory).  A fifth step in registers spills more than it saves:
+// solves of 3,375 to 19,683 nodes take 1 to 4% longer, of 1 to 512 RVEs of sides
+// 6 to 20 0 to 13% (64 of side 20 7.79 against 8.79 ms), and four hold
+// what five do of meshes of this form (fewer than 20,000 nodes) unless their
+// nodes are numbered at random (11,000 nodes against 12,500).  Fewer CTAs a solve also means more solves at once: a
 // chip runs 46 clusters of 3 CTAs, 28 of 5, 15 of 7 to 9, 8 of 11 or 12.
 // FP64 runs at the rate of the FP64 pipe (one warp instruction per 64 cycles
 // and scheduler), not of the storage.  A CTA of 16 warps keeps the first chunk
@@ -40,7 +44,7 @@ template <typename T>
 struct ResShape;
 template <>
 struct ResShape<float> {
-  static constexpr int warps = 16, slots = 4, reg = 5, tm = 7, off = 3, state = 6;
+  static constexpr int warps = 16, slots = 4, reg = 4, tm = 7, off = 3, state = 6;
 };
 template <>
 struct ResShape<double> {
@@ -371,7 +375,11 @@ __device__ __forceinline__ void total3(A (&a)[3], ResShared<T>& sh, int k, int r
 // cycles here and its division 570: 2,200 cycles of every iteration), with
 // alpha = gamma / (delta - gamma (gamma / (gamma_old alpha_old))) so that no
 // squares leave FP32's range; alpha and beta are rounded to FP32 for the
-// update in both.  The reciprocals of the old values are formed off the
+// update in both.  Beside the FP64 scalars of the streamed solves, in 4.7
+// million iterations of RVEs of sides 4 to 24 and meshes of 216 to 97,000
+// nodes: alpha and beta before their rounding differ by at most 2e-6 of an FP32
+// ulp, after it by nothing, and no solve ends at another iteration.  The
+// reciprocals of the old values are formed off the
 // critical path by scalars_next.
 __device__ __forceinline__ ff::dfloat word_ff(u64 w) {
   return ff::fast_two_sum(__uint_as_float((unsigned)w), __uint_as_float((unsigned)(w >> 32)));
