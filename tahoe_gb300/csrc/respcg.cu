@@ -937,8 +937,10 @@ bool resident_plan(const ResRows& R, int elem, int num_sms, const ResLimits& L, 
   P.grid = kmin > max_cluster;
   if (alone) {
     // alone: a cluster while its CTAs hold few chunks each (its exchanges are
-    // short), else every SM
-    const int few = elem == 4 ? 24 : 4;
+    // short), else every SM.  Cluster / grid, us an iteration, by the chunks of
+    // a CTA of the cluster: FP32 16 3.6 / 5.0, 30 4.5 / 4.9, 36 4.9 / 5.2, 51
+    // 5.8 / 5.1; FP64 2 6.6 / 8.4, 5 7.5 / 8.6, 7 9.0 / 8.9, 12 15.1 / 9.3.
+    const int few = elem == 4 ? 40 : 6;
     P.grid = P.grid || (nch + max_cluster - 1) / max_cluster > few;
     const int k = std::max(kmin, std::min(nch, P.grid ? num_sms : max_cluster));
     if (!P.grid) {
