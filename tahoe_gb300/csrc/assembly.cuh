@@ -18,19 +18,17 @@ __device__ __forceinline__ int upper_slot(int a, int b) { return a * 8 - a * (a 
 // destination-sorted order, rows of prescribed dofs zeroed (columns are kept,
 // so a product with a prescribed-increment vector gives the coupling
 // K_fp du_p; PCG vectors are zero at prescribed dofs, so the kept columns
-// never enter the solve).  elem_off: the first element of the instance whose
-// mesh the map describes.
+// never enter the solve).
 template <typename T>
 __device__ __forceinline__ void block_value(int j, uint8_t mI, const int* __restrict__ cptr,
-                                            const int* __restrict__ contrib, const T* __restrict__ Ke, T acc[9],
-                                            int elem_off = 0) {
+                                            const int* __restrict__ contrib, const T* __restrict__ Ke, T acc[9]) {
   using V4 = typename std::conditional<sizeof(T) == 4, float4, double4_32a>::type;
 #pragma unroll
   for (int k = 0; k < 9; ++k) acc[k] = T(0);
   const int c1 = cptr[j + 1];
   for (int c = cptr[j]; c < c1; ++c) {
     const int code = contrib[c];
-    const int e = (code >> 6) + elem_off, a = (code >> 3) & 7, b = code & 7;
+    const int e = code >> 6, a = (code >> 3) & 7, b = code & 7;
     // the element block's three padded rows: one aligned vector load each
     const V4* src = reinterpret_cast<const V4*>(
         Ke + ((long long)e * kSlots + (a <= b ? upper_slot(a, b) : upper_slot(b, a))) * kKeBlock);

@@ -142,3 +142,12 @@ def update_bytes(nnd, s_val):
     to 4 lanes)."""
     s_vec = 4 * s_val
     return nnd * (4 * s_vec + 9 * s_val) + nnd * 4 * s_vec
+
+
+def hybrid_bytes(rows, sms=152):
+    """Bytes an iteration of the hybrid PCG streams for `rows` active nodes, and
+    those of them that come from device memory: chunks of 8 rows, 17 16-byte
+    words a lane, less the 32 chunks an SM keeps in tensor memory; 42 MB of the
+    stream stay in the L2 (hybridpcg.cu)."""
+    streamed = max((rows + 7) // 8 - sms * 32, 0) * 17 * 512
+    return streamed, max(streamed - 42 * (1 << 20), 0)
