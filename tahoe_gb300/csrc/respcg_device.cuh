@@ -250,8 +250,9 @@ struct ResShared {
 // again.  A wait that ran out ends the CTA's others within 64 polls.
 template <typename T>
 __device__ __forceinline__ bool poll_again(ResShared<T>& sh, const WaitLimits& W, int& tries) {
-  if (++tries >= W.polls) sh.abort_flag = 1;
-  return (tries & 63) != 0 || *reinterpret_cast<volatile int*>(&sh.abort_flag) == 0;
+  if (++tries & 63) return true;
+  if (tries >= W.polls) sh.abort_flag = 1;
+  return *reinterpret_cast<volatile int*>(&sh.abort_flag) == 0;
 }
 
 // Totals of three accumulators over every row of the solve, returned to
