@@ -416,9 +416,11 @@ int tg_spmv_release(tg_context* ctx, int per_warp);
  * storage is built on the device on first use after a mesh change and its
  * values are copied from every new assembly.  form = -1 (default): one launch
  * per solve, the rows assembled from the element blocks and kept on the chip,
- * for RVEs and meshes that fit it (in FP64 up to about 25,000 nodes), and in
- * mixed precision up to about 340,000 nodes with the rest of the matrix read
- * from L2 and device memory; the same recurrences as form 1, bitwise
+ * for RVEs and meshes that fit it (in FP64 up to about 25,000 nodes numbered
+ * along the mesh, about 6,000 at random: a CTA holds the column range of its
+ * rows), and in mixed precision from 20,000 to about 340,000 nodes with the rest
+ * of the matrix read from L2 and device memory, where no row has more than 28
+ * blocks; the same recurrences as form 1, bitwise
  * repeatable, different from it by rounding.  Above, and where device memory
  * for it is short: form 3 on meshes of at least one million block nonzeros,
  * form 1 below.  The symmetric format of tg_spmv_symmetric and the

@@ -32,8 +32,8 @@
 //
 // Measured against the streamed kernels (product + vector kernel: 20 us an
 // iteration on a 16^3 FP64 cube, 39 on a 28^3 one; four kernels and 26 us on
-// one RVE of side 8): 9.4, 24.2 and 4.6 us, with no host round trip inside a
-// solve; 4,096 RVEs 540 -> 221 ms with stress, tangent and residuals.  What
+// one RVE of side 8): 9.3, 24.2 and 4.5 us, with no host round trip inside a
+// solve; 4,096 RVEs 540 -> 214 ms with stress, tangent and residuals.  What
 // bounds an iteration: of 12,300 cycles of an RVE of side 15 in a cluster 4,900
 // are the product (shared-memory reads), 1,200 the update and the rest the
 // latency of the exchanges and sums; in FP64 the FP64 pipe.  Whole FP32 meshes
