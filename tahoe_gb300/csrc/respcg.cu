@@ -52,8 +52,8 @@
 #include <exception>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -1165,7 +1165,7 @@ void each_plan(int n, const F& fn) {
   const int more = std::min({7, n / 16, (int)std::thread::hardware_concurrency() - 1});
   try {
     for (int t = 0; t < more; ++t) threads.emplace_back(work);
-  } catch (const std::system_error&) {
+  } catch (...) {
     // no more threads: this one does the rest
   }
   work();
@@ -1327,7 +1327,13 @@ int plan_rows(Context* c, int precision, bool batch, ResMode& M) {
 // memory, keeps nothing: mode -1, and the streamed solves take it.
 int plan_mode(Context* c, int precision, bool batch, ResMode& M) {
   drop_mode(c, M);
-  const int s = plan_rows(c, precision, batch, M);
+  int s = TG_OK;
+  try {
+    s = plan_rows(c, precision, batch, M);
+  } catch (const std::bad_alloc&) {
+    c->err = "no host memory for the plans of the solves on the chip";
+    s = TG_ERR_OOM;
+  }
   if (!s && M.state == 1) return TG_OK;
   drop_mode(c, M);
   M.state = -1;
