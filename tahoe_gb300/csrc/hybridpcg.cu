@@ -612,6 +612,10 @@ int hybrid_plan(Context* c, bool* fits) {
   *fits = false;
   const int n = c->nnd, k = c->num_sms;
   if (c->composed || (int)c->h_coords.size() != 3 * n || n < 8 * k || n > 600000) return TG_OK;
+  auto stream_bytes = [&](long long rows) {
+    return (double)std::max<long long>((rows + 7) / 8 - k * kHybTm * kHybWarps, 1) * kHybVec * 512;
+  };
+  if (stream_bytes(c->neq / 3) > kHybStreamMax) return TG_OK;  // before the nodes are looked at
   hybrid_reset(c);
   cudaStream_t st = c->stream;
   // cells of about eight nodes, at most 2^18
@@ -669,7 +673,7 @@ int hybrid_plan(Context* c, bool* fits) {
     return TG_OK;
   }
   const int nch = (rows + 7) / 8;
-  const double streamed = (double)std::max(nch - k * kHybTm * kHybWarps, 1) * kHybVec * 512;
+  const double streamed = stream_bytes(rows);
   if (streamed > kHybStreamMax) {
     release();
     return TG_OK;

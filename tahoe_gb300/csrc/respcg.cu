@@ -928,6 +928,10 @@ bool resident_plan(const ResRows& R, int elem, int num_sms, const ResLimits& L, 
   P.rows = R.rows;
   P.nchunks = nch;
   if (nch == 0) return false;
+  // a chunk whose columns alone exceed a CTA: no split holds it (shuffled node
+  // numbers; trying every number of CTAs takes half a millisecond)
+  for (int ch = 0; ch < nch; ++ch)
+    if ((size_t)(R.chunk_hi[ch] - R.chunk_lo[ch]) * 4 * elem > cap) return false;
   const int most = elem == 4 ? ResShape<float>::warps * ResShape<float>::slots
                              : ResShape<double>::warps * ResShape<double>::slots;
   int kmin = 0;
